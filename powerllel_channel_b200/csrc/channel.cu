@@ -369,10 +369,10 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
         cudaMemset(*f, 0, sizeof(float) * n);
         return true;
     };
-    // both RK stages in one kernel where the grid tiles: 32 x 8 (FP64
-    // kernel) or 32 x 16 (mixed kernel); else the two stage kernels
-    c->fused_rk = mixed ? rk_mixed_supported(c->sp) : rk_fused_supported(c->sp);
-    if (zn > 1 && !c->fused_rk) {
+    // both RK stages in one kernel: FP64 on every grid, mixed where the grid
+    // tiles by 32 x 16; else the two stage kernels
+    c->fused_rk = !mixed || rk_mixed_supported(c->sp);
+    if (zn > 1 && !(mixed ? c->fused_rk : c->nx % 32 == 0 && c->ny % 8 == 0)) {
         set_error("pl_channel_create_slab: the slab step needs the fused RK kernel: nx % 32 == 0 and ny % 8 == 0 "
                   "(FP64) or ny % 16 == 0 (mixed)");
         return fail();
@@ -416,7 +416,7 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
         }
     }
     c->max_blocks = ((c->nx + 63) / 64) * ((c->ny + 3) / 4) * c->nz;
-    if (c->fused_rk && !mixed && rk_fused_blocks(c->sp) > c->max_blocks) c->max_blocks = rk_fused_blocks(c->sp);
+    if (!mixed && rk_fused_blocks(c->sp) > c->max_blocks) c->max_blocks = rk_fused_blocks(c->sp);
     if (c->fused_rk && mixed && rk_mixed_blocks(c->sp) > c->max_blocks) c->max_blocks = rk_mixed_blocks(c->sp);
     c->rb.max_blocks = c->max_blocks;
     if (cudaMalloc(&c->rb.partial, sizeof(double) * 3 * c->max_blocks) != cudaSuccess ||
@@ -637,8 +637,8 @@ extern "C" int pl_phase_correct_force(pl_channel *c)
     return rc;
 }
 
-// both RK stages in one kernel (out of place) when the grid tiles (32 x 8 FP64,
-// 32 x 16 mixed), else the two stage kernels
+// both RK stages in one kernel (out of place; mixed: when the grid tiles by
+// 32 x 16), else the two stage kernels
 extern "C" int pl_phase_rk(pl_channel *c)
 {
     int rc;

@@ -57,7 +57,6 @@ struct MeanState {
 };
 
 // fused RK1 + RK2 (rk_fused.cu): u -> (uo, vo, wo) out of place
-bool rk_fused_supported(const StepParams &p);
 int rk_fused_blocks(const StepParams &p);
 int launch_rk_fused_fp64(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
                          const StepParams &p, const MeshDev &m, MeanState &ms, cudaStream_t st);
