@@ -12,11 +12,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpowerllel_b200.so")
-SOURCES = ["ppe.cu", "stencil.cu", "rk_fused.cu", "rk_mixed.cu", "channel.cu", "adjoint.cu", "monitor.cu"]
-HEADERS = ["common.cuh", "fft.cuh", "ppe.cuh", "stencil.cuh", "stencil_rhs.cuh", "tmem.cuh", "trid_tables.h", "channel.cuh"]
+SOURCES = ["ppe.cu", "fft_len1.cu", "fft_len2.cu", "fft_len3.cu", "fft_len4.cu", "stencil.cu", "rk_fused.cu", "rk_mixed.cu", "channel.cu", "adjoint.cu", "monitor.cu"]
+HEADERS = ["common.cuh", "fft.cuh", "fft_kernels.cuh", "fft_launch.cuh", "ppe.cuh", "stencil.cuh", "stencil_rhs.cuh", "tmem.cuh", "trid_tables.h", "channel.cuh"]
 
 NVCC_FLAGS = [
-    "-std=c++17", "-O3", "-lineinfo",
+    "-std=c++17", "-O3", "-lineinfo", "--threads", "0",
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC", "-shared",
 ]

@@ -605,7 +605,7 @@ static int phase_rhs_poisson(pl_channel *c)
         const int rc = ppe_xfwd_div<float>(&c->ppe, d, c->r32, c->plane_part, c->stream);
         if (rc < 0) return -1;
         if (rc == 0) {
-            if (launch_plane_sums(c->plane_part, c->sp.ny / 2, c->nz, c->mode0, c->stream)) return -1;
+            if (launch_plane_sums(c->plane_part, ppe_xdiv_parts(&c->ppe), c->nz, c->mode0, c->stream)) return -1;
             channel_mark(c, "rhs_xfft");
             const PressureUpdate pu = mixed_pressure_update(c);
             c->p_stale = true;
@@ -948,7 +948,7 @@ extern "C" int pl_slab_rhs_sweep(pl_channel *c)
         return is_mixed(c) ? ppe_slab_forward<float>(&c->ppe, c->r32, c->stream, c->mode0)
                            : ppe_slab_forward<double>(&c->ppe, c->p, c->stream, nullptr);
     }
-    if (is_mixed(c) && launch_plane_sums(c->plane_part, c->sp.ny / 2, c->nz, c->mode0, c->stream)) return -1;
+    if (is_mixed(c) && launch_plane_sums(c->plane_part, ppe_xdiv_parts(&c->ppe), c->nz, c->mode0, c->stream)) return -1;
     channel_mark(c, "rhs_xfft");
     return is_mixed(c) ? ppe_slab_forward_from_x<float>(&c->ppe, c->r32, c->stream, c->mode0)
                        : ppe_slab_forward_from_x<double>(&c->ppe, c->p, c->stream, nullptr);

@@ -1,0 +1,6 @@
+// transform kernels of the line lengths in PL_FFT_LEN3
+#include "fft_kernels.cuh"
+
+namespace pl {
+PL_FFT_LEN3(PL_FFT_INSTANTIATE)
+} // namespace pl

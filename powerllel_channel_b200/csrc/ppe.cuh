@@ -97,10 +97,11 @@ struct DivIn {
 };
 // Forward x transform of rhs = div(u)/dt computed on the fly, into the
 // interior-only array out (T = double: the FP64 solve's, float: the mixed
-// one's); part (optional, nz * ny/2 doubles): per line pair, the FP64 sum of
-// its rhs values.  Returns 1 (nothing launched) where the fused kernel does
+// one's); part (optional, nz * ppe_xdiv_parts doubles, at most nz * ny/2): the
+// FP64 sums of the rhs values of each group of lines.  Returns 1 (nothing launched) where the fused kernel does
 // not apply: nx not a compile-time transform length.
 template <typename T> int ppe_xfwd_div(Ppe *s, const DivIn &d, T *out, double *part, cudaStream_t st);
+int ppe_xdiv_parts(const Ppe *s); // partial sums per plane that ppe_xfwd_div writes
 // FP64 solve when d_var already holds the forward x transform
 int ppe_solve_fp64_from_x(Ppe *s, double *d_var, cudaStream_t st);
 

@@ -1,0 +1,91 @@
+"""The Poisson solve and the step over every compiled line length, in x and in y, with column
+heights around the groups of eight rows that the tridiagonal sweeps work in."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [16, 18, 24, 32, 36, 48, 54, 72, 96, 108, 128, 144, 162, 216, 288, 324, 432, 486, 576, 648, 864, 972]
+
+
+def rhs_and_reference(O, nx, ny, nz, nparts=0):
+    g = O.Grid(nx, ny, nz, stretch=1.6)
+    r = np.random.default_rng(nx * 1000 + ny + nz).standard_normal((nz, ny, nx))
+    wgt = g.dzf_global[1:-1]
+    r -= (r.mean(axis=(1, 2)) * wgt).sum() / wgt.sum()
+    var = np.zeros(g.shape)
+    var[1:-1, 1:-1, 1:-1] = r
+    O.PPE(nx, ny, nz, g.g.dx, g.g.dy, g.dzf_global, nparts=nparts).execute(var)
+    p = var[1:-1, 1:-1, 1:-1]
+    return g, r, p - p.mean()
+
+
+def solve(plb, g, r, precision, nparts=0):
+    import torch
+    nz, ny, nx = r.shape
+    s = plb.DevicePoissonSolver(nx, ny, nz, g.g.dx, g.g.dy, g.dzf_global, nparts=nparts, precision=precision)
+    x = torch.tensor(r, dtype=torch.float64 if precision == plb.PL_FP64 else torch.float32, device="cuda")
+    s.solve(x)
+    torch.cuda.synchronize()
+    p = x.cpu().numpy().astype(np.float64)
+    return p - p.mean()
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("n", LENGTHS)
+def test_solve_by_line_length(gpu, oracle_mod, n, precision, tol):
+    """x of length n over y of the next length and the other way round (ny/2 not a multiple of the
+    lines a group holds; odd column counts), at a height of ten rows.  Tolerances as for the
+    other lengths: the FP64 bar, and FP32 transforms."""
+    plb, O = gpu, oracle_mod
+    other = LENGTHS[(LENGTHS.index(n) + 1) % 6]
+    for nx, ny in ((n, other), (other, n)):
+        g, r, ref = rhs_and_reference(O, nx, ny, 10)
+        got = solve(plb, g, r, plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED)
+        assert np.abs(got - ref).max() < tol * np.abs(ref).max(), (nx, ny)
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("nz", [2, 6, 14, 22, 150, 250, 254, 258, 274, 306])
+def test_solve_by_column_height(gpu, oracle_mod, nz, precision, tol):
+    """Heights that the groups of eight rows do not divide, up to and beyond the 256 rows that
+    tensor memory holds; 162 columns a row, so the last CTA is partly empty."""
+    plb, O = gpu, oracle_mod
+    g, r, ref = rhs_and_reference(O, 162, 16, nz)
+    got = solve(plb, g, r, plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED)
+    assert np.abs(got - ref).max() < tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("nz,nparts", [(64, 4), (96, 6), (120, 5), (128, 8), (192, 3)])
+def test_pdd_by_partition_size(gpu, oracle_mod, nz, nparts, precision, tol):
+    """Partitions of 8, 16, 24 and 64 rows: loads of 8 and of 16 rows."""
+    plb, O = gpu, oracle_mod
+    g, r, ref = rhs_and_reference(O, 54, 18, nz, nparts)
+    got = solve(plb, g, r, plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED, nparts)
+    assert np.abs(got - ref).max() < tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny,nz", [(16, 6, 4), (54, 18, 14), (96, 24, 22), (162, 16, 10), (324, 8, 6)])
+def test_step_matches_phases(gpu, precision, nx, ny, nz):
+    """calcRHS inside the forward x transform (several lines per group at short lengths, the
+    last group of a plane partly filled) against calcRHS as its own kernel: FP64 bit for bit;
+    mixed to 1e-11, the plane sums being added in another order."""
+    plb = gpu
+    cfg = plb.ChannelConfig(nx=nx, ny=ny, nz=nz, stretch_ratio=1.5, re_tau=180.0,
+                            precision=plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED)
+    a, b = plb.Channel(cfg), plb.Channel(cfg)
+    for ch in (a, b):
+        ch.init_flow(5, 0.1)
+    for _ in range(4):
+        a.step(1)
+        for ph in ("rk", "calc_rhs", "poisson", "correct_force"):
+            b.phase(ph)
+    for x, y in zip(a.get_fields()[:3], b.get_fields()[:3]):
+        if precision == "fp64":
+            assert np.array_equal(x, y)
+        else:
+            assert np.abs(x - y).max() < 1e-11 * np.abs(y).max()
+    a.close()
+    b.close()
