@@ -311,7 +311,7 @@ struct TtmColumn {
 // GAUGE: the (0,0) column (mode0 given) takes x[nz-1] = 0, the free
 // constant of the singular whole-column system; a slab's partition system is
 // regular and solves that column from the plane sums without it.
-template <typename T, bool TALL, typename TO = T, bool GAUGE = true>
+template <typename T, bool TALL, typename TO = T, bool GAUGE = true, bool RAGGED = false>
 __global__ void __launch_bounds__(TTM_THREADS, 1)
     k_thomas_tmem(const T *xin, TO *xout, double *xsc, TridDev t, const double *mode0, int rounds, uint32_t tcols)
 {
@@ -324,10 +324,12 @@ __global__ void __launch_bounds__(TTM_THREADS, 1)
     uint32_t *tslot = reinterpret_cast<uint32_t *>(csh + TTM_MAX_NZ);
     double *sring = sizeof(T) == 8 ? reinterpret_cast<double *>(xring) : csh + TTM_MAX_NZ + 2; // HBM rows, bwd
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int nz = t.nz, ngf = nz / G, per_round = 2 * ngf;
+    // RAGGED: the top group reaches nze - nz rows past the column, which are
+    // neither copied nor stored and count as zero in the back substitution
+    const int nz = t.nz, ngf = RAGGED ? (nz + G - 1) / G : nz / G, nze = RAGGED ? ngf * G : nz, per_round = 2 * ngf;
     // rows [kb, kt) live in the HBM scratch (none when nz <= TTM_TM_ROWS);
     // row k < kb sits at TMEM cell 2k, row k >= kt at 2 (kb + k - kt)
-    const int kb = TALL ? TTM_TM_ROWS - TTM_TOP_ROWS : nz, kt = TALL ? nz - TTM_TOP_ROWS : nz;
+    const int kb = TALL ? TTM_TM_ROWS - TTM_TOP_ROWS : nze, kt = TALL ? nze - TTM_TOP_ROWS : nze;
     auto in_hbm = [&](int k0) { return TALL && k0 >= kb && k0 < kt; }; // k0: first row of an 8-row group
     auto tcell = [&](int k0) { return TALL ? 2 * (k0 < kb ? k0 : kb + k0 - kt) : 2 * k0; };
     const size_t stride = (size_t)t.nx * t.ny, cstride = (size_t)t.ncx * t.ncy;
@@ -358,8 +360,8 @@ __global__ void __launch_bounds__(TTM_THREADS, 1)
     int ir = 0, ig = 0, islot = 0;
     TtmColumn ic = column(0);
     const T *xsrc = xin + ic.col;
-    const double *msrc = t.mult + ic.cls, *rsrc = t.rb + ic.cls + (size_t)(nz - 1) * cstride;
-    const double *ssrc = xsc + ic.col + (size_t)(nz - 1) * stride;
+    const double *msrc = t.mult + ic.cls, *rsrc = t.rb + ic.cls + (size_t)(nze - 1) * cstride;
+    const double *ssrc = xsc + ic.col + (size_t)(nze - 1) * stride;
     auto issue_next = [&]() {
         if (ir < rounds) {
             double *cdst = cring + islot * G * NT + tid;
@@ -369,6 +371,7 @@ __global__ void __launch_bounds__(TTM_THREADS, 1)
                 if (ic.valid) {
 #pragma unroll
                     for (int u = 0; u < G; u++) {
+                        if (RAGGED && ig * G + u >= nz) break;
                         cp_async_8(cdst + u * NT, msrc);
                         if (z)
                             cp_async_8(zring + islot * G + u, mode0 + ig * G + u);
@@ -381,11 +384,11 @@ __global__ void __launch_bounds__(TTM_THREADS, 1)
                     }
                 }
             } else if (ic.valid) {
-                const bool hb = in_hbm(nz - (ig - ngf + 1) * G);
+                const bool hb = in_hbm(nze - (ig - ngf + 1) * G);
                 double *sdst = sring + islot * G * NT + tid;
 #pragma unroll
                 for (int u = 0; u < G; u++) {
-                    cp_async_8(cdst + u * NT, rsrc);
+                    if (!RAGGED || nze - 1 - (ig - ngf) * G - u < nz) cp_async_8(cdst + u * NT, rsrc);
                     rsrc -= cstride;
                     if constexpr (TALL) {
                         if (hb) cp_async_8(sdst + u * NT, ssrc);
@@ -399,8 +402,8 @@ __global__ void __launch_bounds__(TTM_THREADS, 1)
                     ic = column(ir);
                     xsrc = xin + ic.col;
                     msrc = t.mult + ic.cls;
-                    rsrc = t.rb + ic.cls + (size_t)(nz - 1) * cstride;
-                    ssrc = xsc + ic.col + (size_t)(nz - 1) * stride;
+                    rsrc = t.rb + ic.cls + (size_t)(nze - 1) * cstride;
+                    ssrc = xsc + ic.col + (size_t)(nze - 1) * stride;
                 }
             }
         }
@@ -451,9 +454,9 @@ __global__ void __launch_bounds__(TTM_THREADS, 1)
         // (:346-356); at k = nz-1, with x_{nz} = 0, it is x /= b (:332-344),
         // and the (0,0) mode takes the gauge x[nz-1] = 0 there
         xp = 0.0;
-        TO *dst = xout + cc.col + (size_t)(nz - 1) * stride;
+        TO *dst = xout + cc.col + (size_t)(nze - 1) * stride;
         for (int h = 0; h < ngf; h++) {
-            const int ktop = nz - 1 - h * G; // rows ktop, ktop-1, ..., ktop-G+1
+            const int ktop = nze - 1 - h * G; // rows ktop, ktop-1, ..., ktop-G+1
             uint32_t v[2 * G];
             const bool hb = in_hbm(ktop - G + 1); // warp-uniform
             if (!hb) {
@@ -468,7 +471,11 @@ __global__ void __launch_bounds__(TTM_THREADS, 1)
                 rv[u] = cs[u * NT];
                 cv[u] = csh[ktop - u];
             }
-            if (GAUGE && zr && tid == 0 && h == 0) rv[0] = 0.0;
+            if (GAUGE && zr && tid == 0 && h == 0) {
+#pragma unroll
+                for (int u = 0; u < (RAGGED ? G : 1); u++)
+                    if (!RAGGED || ktop - u == nz - 1) rv[u] = 0.0;
+            }
             issue_next();
             if (!hb) tmem_wait_ld(v);
             const double *ss = sring + slot * G * NT + tid;
@@ -476,8 +483,9 @@ __global__ void __launch_bounds__(TTM_THREADS, 1)
             for (int u = 0; u < G; u++) {
                 const int i = G - 1 - u;
                 const double x = hb ? ss[u * NT] : __hiloint2double((int)v[2 * i + 1], (int)v[2 * i]);
-                xp = (x - cv[u] * xp) * rv[u];
-                if (cc.valid) *dst = (TO)xp;
+                const bool past = RAGGED && ktop - u >= nz;
+                xp = past ? 0.0 : (x - cv[u] * xp) * rv[u];
+                if (cc.valid && !past) *dst = (TO)xp;
                 dst -= stride;
             }
             slot = (slot + 1 == NS) ? 0 : slot + 1;
@@ -1671,7 +1679,7 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
         return 0;
     }
     double *xs = (sizeof(T) == 8 && s->nparts == 0) ? reinterpret_cast<double *>(x) : s->d_scratch;
-    if (s->nparts == 0 && s->nz % TTM_G == 0 && s->nz <= TTM_MAX_NZ &&
+    if (s->nparts == 0 && s->nz <= TTM_MAX_NZ &&
         (s->nz <= TTM_TM_ROWS || sizeof(T) == 8 || s->d_scratch != nullptr)) {
         // swept values in TMEM (taller columns partly in the HBM scratch: in
         // place for FP64, the FP64 sweep scratch for FP32): one 128-thread CTA
@@ -1681,17 +1689,13 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
         const int ctas = std::max(1, std::min(sm_count(), (ncol + TTM_THREADS - 1) / TTM_THREADS));
         const int rounds = (ncol + ctas * TTM_THREADS - 1) / (ctas * TTM_THREADS);
         uint32_t tcols = 32;
-        while (tcols < 2u * (uint32_t)std::min(s->nz, TTM_TM_ROWS)) tcols *= 2;
+        while (tcols < 2u * (uint32_t)std::min((s->nz + TTM_G - 1) / TTM_G * TTM_G, TTM_TM_ROWS)) tcols *= 2;
         double *xsc = sizeof(T) == 8 ? reinterpret_cast<double *>(x) : s->d_scratch;
-        if (s->nz > TTM_TM_ROWS) {
-            PL_CUDA_TRY(
-                cudaFuncSetAttribute(k_thomas_tmem<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-            k_thomas_tmem<T, true><<<ctas, TTM_THREADS, shm, st>>>(x, x, xsc, t, mode0, rounds, tcols);
-        } else {
-            PL_CUDA_TRY(
-                cudaFuncSetAttribute(k_thomas_tmem<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-            k_thomas_tmem<T, false><<<ctas, TTM_THREADS, shm, st>>>(x, x, xsc, t, mode0, rounds, tcols);
-        }
+        const bool tall = s->nz > TTM_TM_ROWS, ragged = s->nz % TTM_G != 0;
+        auto kern = tall ? (ragged ? k_thomas_tmem<T, true, T, true, true> : k_thomas_tmem<T, true>)
+                         : (ragged ? k_thomas_tmem<T, false, T, true, true> : k_thomas_tmem<T, false>);
+        PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+        kern<<<ctas, TTM_THREADS, shm, st>>>(x, x, xsc, t, mode0, rounds, tcols);
     } else if (s->nparts == 0) {
         k_thomas<T><<<grid, 128, 0, st>>>(x, xs, x, t, mode0);
     } else if (s->nparts <= 32) {
