@@ -1103,20 +1103,20 @@ constexpr int PTM_G = 8;
 
 __host__ __device__ constexpr int pdd_tm_static_smem() { return 2 * 8 * 32 * 8 + 16; }
 
-template <typename T>
+template <typename T, int B>
 __global__ void __launch_bounds__(256) k_pdd_tm(const T *xin, T *xout, TridDev t, PddDev p, const double *mode0,
                                                 int kmax, uint32_t tcols)
 {
-    constexpr int G = PTM_G;
+    constexpr int G = PTM_G, H = B / G;
     __shared__ double edge[2][8][32]; // [first / last local value][partition][column]
     __shared__ uint32_t tslot;
     const int cx = threadIdx.x, m = threadIdx.y;
     const int q = blockIdx.x * 32 + cx, ncol = t.nx * t.ny;
     const bool valid = q < ncol;
-    const int qq = valid ? q : 0, px = qq % t.nx, py = qq / t.nx;
-    const size_t col = (size_t)qq, stride = (size_t)t.nx * t.ny;
+    const int qq = valid ? q : 0, px = qq % t.nx, py = trid_pair_row(qq / t.nx, t.ny);
+    const size_t col = (size_t)px + (size_t)t.nx * py, stride = (size_t)t.nx * t.ny;
     const size_t cls = trid_class(px, py, t), cstride = (size_t)t.ncx * t.ncy;
-    const int k0 = p.kst[m], ke = p.ksz[m], ng = ke / G;
+    const int k0 = p.kst[m], ke = p.ksz[m], ng = ke / B;
     const bool z = mode0 != nullptr && valid && col == 0; // mixed path: the (0,0) column from the plane sums
 
     if (m == 0) tmem_alloc(&tslot, tcols);
@@ -1129,49 +1129,54 @@ __global__ void __launch_bounds__(256) k_pdd_tm(const T *xin, T *xout, TridDev t
     // multiplier is 0 at its first row)
     double xp = 0.0;
     for (int g = 0; g < ng; g++) {
-        double xv[G], mv[G];
+        double xv[B], mv[B];
 #pragma unroll
-        for (int u = 0; u < G; u++) {
-            const int k = k0 + g * G + u;
+        for (int u = 0; u < B; u++) {
+            const int k = k0 + g * B + u;
             xv[u] = z ? mode0[k] : (double)xin[col + (size_t)k * stride];
             mv[u] = __ldg(t.mult + cls + (size_t)k * cstride);
         }
-        uint32_t v[2 * G];
 #pragma unroll
-        for (int u = 0; u < G; u++) {
-            xp = xv[u] - mv[u] * xp;
-            v[2 * u] = (uint32_t)__double2loint(xp);
-            v[2 * u + 1] = (uint32_t)__double2hiint(xp);
+        for (int h = 0; h < H; h++) {
+            uint32_t v[2 * G];
+#pragma unroll
+            for (int u = 0; u < G; u++) {
+                xp = xv[h * G + u] - mv[h * G + u] * xp;
+                v[2 * u] = (uint32_t)__double2loint(xp);
+                v[2 * u + 1] = (uint32_t)__double2hiint(xp);
+            }
+            __syncwarp();
+            tmem_st16(tb + 2 * (g * B + h * G), v);
         }
-        __syncwarp();
-        tmem_st16(tb + 2 * g * G, v);
     }
     tmem_wait_st();
     // back substitution (:332-356): x = (x - c x_{k+1}) / b, with x_{k+1} = 0
     // above the partition's last row; the local solution replaces the swept rows
     double w = 0.0, first = 0.0, last = 0.0;
     for (int g = ng - 1; g >= 0; g--) {
-        uint32_t v[2 * G];
-        __syncwarp();
-        tmem_ld16_start(tb + 2 * g * G, v);
-        double rv[G], cv[G];
+        double rv[B];
 #pragma unroll
-        for (int u = 0; u < G; u++) {
-            const int k = k0 + g * G + u;
-            rv[u] = __ldg(t.rb + cls + (size_t)k * cstride);
-            cv[u] = __ldg(t.c + k);
-        }
-        tmem_wait_ld(v);
+        for (int u = 0; u < B; u++) rv[u] = __ldg(t.rb + cls + (size_t)(k0 + g * B + u) * cstride);
 #pragma unroll
-        for (int u = G - 1; u >= 0; u--) {
-            const double s = __hiloint2double((int)v[2 * u + 1], (int)v[2 * u]);
-            w = (s - cv[u] * w) * rv[u];
-            if (g == ng - 1 && u == G - 1) last = w;
-            v[2 * u] = (uint32_t)__double2loint(w);
-            v[2 * u + 1] = (uint32_t)__double2hiint(w);
+        for (int h = H - 1; h >= 0; h--) {
+            uint32_t v[2 * G];
+            __syncwarp();
+            tmem_ld16_start(tb + 2 * (g * B + h * G), v);
+            double cv[G];
+#pragma unroll
+            for (int u = 0; u < G; u++) cv[u] = __ldg(t.c + k0 + g * B + h * G + u);
+            tmem_wait_ld(v);
+#pragma unroll
+            for (int u = G - 1; u >= 0; u--) {
+                const double s = __hiloint2double((int)v[2 * u + 1], (int)v[2 * u]);
+                w = (s - cv[u] * w) * rv[h * G + u];
+                if (g == ng - 1 && h == H - 1 && u == G - 1) last = w;
+                v[2 * u] = (uint32_t)__double2loint(w);
+                v[2 * u + 1] = (uint32_t)__double2hiint(w);
+            }
+            __syncwarp();
+            tmem_st16(tb + 2 * (g * B + h * G), v);
         }
-        __syncwarp();
-        tmem_st16(tb + 2 * g * G, v);
     }
     first = w;
     tmem_wait_st();
@@ -1197,22 +1202,26 @@ __global__ void __launch_bounds__(256) k_pdd_tm(const T *xin, T *xout, TridDev t
     if (m + 1 < p.nparts) iface(m, y2, unused);
     // correction x = x_local - v y1 - w y2 (:452-464)
     for (int g = 0; g < ng; g++) {
-        uint32_t v[2 * G];
-        __syncwarp();
-        tmem_ld16_start(tb + 2 * g * G, v);
-        double vv[G], wv[G];
+        double vv[B], wv[B];
 #pragma unroll
-        for (int u = 0; u < G; u++) {
-            const size_t gc = cls + (size_t)(k0 + g * G + u) * cstride;
+        for (int u = 0; u < B; u++) {
+            const size_t gc = cls + (size_t)(k0 + g * B + u) * cstride;
             vv[u] = __ldg(p.v + gc);
             wv[u] = __ldg(p.w + gc);
         }
-        tmem_wait_ld(v);
-        if (valid) {
 #pragma unroll
-            for (int u = 0; u < G; u++) {
-                const double x = __hiloint2double((int)v[2 * u + 1], (int)v[2 * u]);
-                xout[col + (size_t)(k0 + g * G + u) * stride] = (T)(x - vv[u] * y1 - wv[u] * y2);
+        for (int h = 0; h < H; h++) {
+            uint32_t v[2 * G];
+            __syncwarp();
+            tmem_ld16_start(tb + 2 * (g * B + h * G), v);
+            tmem_wait_ld(v);
+            if (valid) {
+#pragma unroll
+                for (int u = 0; u < G; u++) {
+                    const double x = __hiloint2double((int)v[2 * u + 1], (int)v[2 * u]);
+                    xout[col + (size_t)(k0 + g * B + h * G + u) * stride] =
+                        (T)(x - vv[h * G + u] * y1 - wv[h * G + u] * y2);
+                }
             }
         }
     }
@@ -1702,12 +1711,13 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
         PddDev p{};
         p.nparts = s->nparts;
         int kmax = 0;
-        bool groups = true;
+        bool groups = true, groups2 = true;
         for (int m = 0; m < s->nparts; m++) {
             p.kst[m] = s->kst[m];
             p.ksz[m] = s->ksz[m];
             kmax = std::max(kmax, s->ksz[m]);
             groups = groups && s->ksz[m] >= PTM_G && s->ksz[m] % PTM_G == 0;
+            groups2 = groups2 && s->ksz[m] % (2 * PTM_G) == 0;
         }
         p.v = s->d_v;
         p.w = s->d_w;
@@ -1721,10 +1731,12 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
             while (tcols < (uint32_t)cells) tcols *= 2;
             const int per_sm = std::max(1, std::min(512 / (int)tcols, 2048 / (32 * s->nparts)));
             const int dyn = std::max(0, 233472 / per_sm - 1024 - pdd_tm_static_smem() - 512);
+            // loads of 16 rows in flight where the partitions allow, else 8
+            auto kern = groups2 ? k_pdd_tm<T, 2 * PTM_G> : k_pdd_tm<T, PTM_G>;
             if (dyn > 48 * 1024)
-                PL_CUDA_TRY(cudaFuncSetAttribute(k_pdd_tm<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-            k_pdd_tm<T><<<(ncol + 31) / 32, dim3(32, s->nparts), dyn, st>>>(x, x, t, p, sizeof(T) == 4 ? mode0 : nullptr,
-                                                                             kmax, tcols);
+                PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+            kern<<<(ncol + 31) / 32, dim3(32, s->nparts), dyn, st>>>(x, x, t, p, sizeof(T) == 4 ? mode0 : nullptr, kmax,
+                                                                      tcols);
         } else {
             k_pdd_par<T><<<(ncol + 31) / 32, dim3(32, s->nparts), 0, st>>>(x, s->d_scratch, x, t, p,
                                                                           sizeof(T) == 4 ? mode0 : nullptr);
