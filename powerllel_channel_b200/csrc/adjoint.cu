@@ -37,7 +37,7 @@ using namespace pl;
 
 namespace {
 
-constexpr int SUM_PARTS = 8; // partial sums per level in the plane reductions
+constexpr int SUM_PARTS = MON_PARTS; // partial sums per level in the plane reductions
 
 dim3 adj_block() { return dim3(64, 4, 1); }
 dim3 adj_grid(const StepParams &p) { return dim3((p.nx + 63) / 64, (p.ny + 3) / 4, p.nz); }
@@ -192,15 +192,23 @@ __global__ void __launch_bounds__(256) k_level_sums(const double *__restrict__ a
     }
 }
 
-// out[c] = (accumulate ? out[c] : 0) + coef * sum of the level partials, in k order
-__global__ void k_sums_finish(const double *__restrict__ part, int nz, double coef, int accumulate,
-                              double *__restrict__ out)
+// out[c] = (accumulate ? out[c] : 0) + coef * sum of the level partials, one
+// component per block, as a tree of fixed order (three threads adding the
+// 1,024 partials of 128 levels one after the other waited on every load)
+__global__ void __launch_bounds__(256) k_sums_finish(const double *__restrict__ part, int nz, double coef,
+                                                     int accumulate, double *__restrict__ out)
 {
-    const int c = threadIdx.x;
-    if (c >= 3) return;
+    __shared__ double sh[256];
+    const int c = blockIdx.x, t = threadIdx.x;
     double s = 0.0;
-    for (int x = 0; x < nz * SUM_PARTS; x++) s += part[(size_t)x * 3 + c];
-    out[c] = (accumulate ? out[c] : 0.0) + coef * s;
+    for (int x = t; x < nz * SUM_PARTS; x += 256) s += part[(size_t)x * 3 + c];
+    sh[t] = s;
+    __syncthreads();
+    for (int h = 128; h > 0; h >>= 1) {
+        if (t < h) sh[t] += sh[t + h];
+        __syncthreads();
+    }
+    if (t == 0) out[c] = (accumulate ? out[c] : 0.0) + coef * sh[0];
 }
 
 // forceVel^T and division by the cell volumes: z = W^-1 (xbar - c_k S e_x),
@@ -268,20 +276,41 @@ __global__ void __launch_bounds__(256) k_adj_seed(const double *__restrict__ u, 
     aw[g] = (k == p.nz) ? 0.0 : dxdy / __ldg(m.dzc_inv + k) * w[g];
 }
 
+// The adjoint's device memory, kept with the channel from its first use (a
+// program takes gradients one after the other): allocating, clearing and
+// freeing it on every call cost as much as several steps at 256x192x128.  The
+// ghost planes of xa, y2 and y1 are zero from their allocation on.
 struct AdjWork {
-    std::vector<double *> owned;
-    double *ck = nullptr, *seg = nullptr;           // checkpoints, segment states (3 fields each)
+    double *ck = nullptr, *seg = nullptr;               // checkpoints, segment states (3 fields each)
     double *xa = nullptr, *y2 = nullptr, *y1 = nullptr; // adjoint fields (3 fields each)
     double *part = nullptr, *scal = nullptr, *fbar = nullptr;
-    ~AdjWork()
+    size_t nck = 0, nseg = 0; // states that ck and seg hold
+    void release()
     {
-        for (double *p : owned) cudaFree(p);
+        for (double *p : {ck, seg, xa, y2, y1, part}) cudaFree(p);
+        *this = AdjWork();
     }
-    bool alloc(double **p, size_t n, cudaStream_t st)
+    bool reserve(size_t nck_, size_t nseg_, const pl_channel *c)
     {
-        if (cudaMalloc(p, sizeof(double) * n) != cudaSuccess) return false;
-        owned.push_back(*p);
-        return cudaMemsetAsync(*p, 0, sizeof(double) * n, st) == cudaSuccess;
+        const size_t fields = 3 * c->nf * sizeof(double), sums = (3 * SUM_PARTS * (size_t)c->nz + 16) * sizeof(double);
+        auto grow = [&](double **p, size_t &have, size_t need) {
+            if (have >= need) return true;
+            cudaFree(*p);
+            *p = nullptr;
+            have = 0;
+            if (cudaMalloc(p, fields * need) != cudaSuccess) return false;
+            have = need;
+            return true;
+        };
+        if (!grow(&ck, nck, nck_) || !grow(&seg, nseg, nseg_)) return false;
+        for (double **p : {&xa, &y2, &y1})
+            if (!*p && (cudaMalloc(p, fields) != cudaSuccess ||
+                        cudaMemsetAsync(*p, 0, fields, c->stream) != cudaSuccess))
+                return false;
+        if (!part && cudaMalloc(&part, sums) != cudaSuccess) return false;
+        scal = part + 3 * SUM_PARTS * (size_t)c->nz;
+        fbar = scal + 4;
+        return cudaMemsetAsync(scal, 0, 16 * sizeof(double), c->stream) == cudaSuccess;
     }
 };
 
@@ -294,7 +323,7 @@ int level_sums(int mode, const double *a, const double *b, const double *c, cons
     else
         k_level_sums<1><<<g, 256, 0, ch->stream>>>(a, b, c, ch->sp, ch->m, part);
     PL_CHECK_LAUNCH();
-    k_sums_finish<<<1, 32, 0, ch->stream>>>(part, ch->nz, coef, accumulate, out);
+    k_sums_finish<<<3, 256, 0, ch->stream>>>(part, ch->nz, coef, accumulate, out);
     PL_CHECK_LAUNCH();
     return 0;
 }
@@ -345,6 +374,14 @@ int adjoint_step(pl_channel *c, const double *xu, const double *xv, const double
 
 } // namespace
 
+void pl::adjoint_free(pl_channel *c)
+{
+    if (!c->adj) return;
+    static_cast<AdjWork *>(c->adj)->release();
+    delete static_cast<AdjWork *>(c->adj);
+    c->adj = nullptr;
+}
+
 extern "C" int pl_channel_set_body_force(pl_channel *c, const double f[3])
 {
     if (c->cfg.precision != PL_FP64 && (f[0] != 0.0 || f[1] != 0.0 || f[2] != 0.0)) {
@@ -357,14 +394,11 @@ extern "C" int pl_channel_set_body_force(pl_channel *c, const double f[3])
 
 extern "C" int pl_channel_kinetic_energy(pl_channel *c, double *ke)
 {
-    double *part = nullptr, *out = nullptr;
-    PL_CUDA_TRY(cudaMalloc(&part, sizeof(double) * (3 * SUM_PARTS * (size_t)c->nz + 4)));
-    out = part + 3 * SUM_PARTS * (size_t)c->nz;
-    int rc = level_sums(1, c->u, c->v, c->w, c, part, 1.0, 0, out);
+    double *out = c->d_mon;
+    int rc = level_sums(1, c->u, c->v, c->w, c, c->d_mon + MON_OUT, 1.0, 0, out);
     double h[3] = {0, 0, 0};
     if (!rc && cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess) rc = -1;
     if (!rc && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = -1;
-    cudaFree(part);
     if (rc) {
         set_error("pl_channel_kinetic_energy: device error");
         return -1;
@@ -395,15 +429,14 @@ extern "C" int pl_adjoint_ke_gradient(pl_channel *c, int nsteps, int every, doub
     cudaStream_t st = c->stream;
     const int nck = (nsteps + every - 1) / every;
     const int nseg = std::min(every, std::max(nsteps, 1));
-    AdjWork W;
-    if (!W.alloc(&W.ck, 3 * nf * (size_t)std::max(nck, 1), st) || !W.alloc(&W.seg, 3 * nf * (size_t)nseg, st) ||
-        !W.alloc(&W.xa, 3 * nf, st) || !W.alloc(&W.y2, 3 * nf, st) || !W.alloc(&W.y1, 3 * nf, st) ||
-        !W.alloc(&W.part, 3 * SUM_PARTS * (size_t)c->nz + 16, st)) {
+    if (!c->adj) c->adj = new AdjWork();
+    AdjWork &W = *static_cast<AdjWork *>(c->adj);
+    if (!W.reserve(std::max(nck, 1), nseg, c)) {
+        W.release();
+        (void)cudaGetLastError();
         set_error("pl_adjoint_ke_gradient: out of device memory for checkpoints and adjoint fields");
         return -1;
     }
-    W.scal = W.part + 3 * SUM_PARTS * (size_t)c->nz;
-    W.fbar = W.scal + 4;
     auto state = [&](double *base, int slot) { return base + 3 * nf * (size_t)slot; };
 
     // forward sweep with checkpoints

@@ -264,7 +264,9 @@ static void channel_free(pl_channel *c)
     cudaFree(c->rb.partial);
     cudaFree(c->rb.scalar);
     cudaFree(c->d_diag);
-    cudaFree(c->d_loc);
+    cudaFree(c->d_mon);
+    cudaFree(c->d_mon_count);
+    adjoint_free(c);
     cudaFree(c->d_dpart);
     cudaFree(c->d_dipart);
     ppe_destroy(&c->ppe);
@@ -421,8 +423,9 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
     c->rb.max_blocks = c->max_blocks;
     if (cudaMalloc(&c->rb.partial, sizeof(double) * 3 * c->max_blocks) != cudaSuccess ||
         cudaMalloc(&c->rb.scalar, sizeof(double) * 8) != cudaSuccess ||
-        cudaMalloc(&c->d_diag, sizeof(double) * 4) != cudaSuccess ||
-        cudaMalloc(&c->d_loc, sizeof(int) * 8) != cudaSuccess ||
+        cudaMalloc(&c->d_diag, sizeof(double) * 8) != cudaSuccess ||
+        cudaMalloc(&c->d_mon, sizeof(double) * (MON_OUT + 64 + 3 * MON_PARTS * (size_t)c->nz)) != cudaSuccess ||
+        cudaMalloc(&c->d_mon_count, sizeof(unsigned int)) != cudaSuccess ||
         cudaMalloc(&c->d_dpart, sizeof(double) * 3 * c->max_blocks) != cudaSuccess ||
         cudaMalloc(&c->d_dipart, sizeof(long long) * 2 * c->max_blocks) != cudaSuccess ||
         cudaMalloc(&c->ms.partial, sizeof(double) * c->max_blocks) != cudaSuccess ||
@@ -431,6 +434,7 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
         return fail();
     }
     cudaMemset(c->ms.counter, 0, sizeof(unsigned int));
+    cudaMemset(c->d_mon_count, 0, sizeof(unsigned int));
     cudaMemset(c->rb.scalar, 0, sizeof(double) * 8);
     c->ms.scalar = c->rb.scalar;
     c->ms.max_blocks = c->max_blocks;
@@ -717,14 +721,15 @@ extern "C" int pl_channel_synchronize(pl_channel *c)
 
 extern "C" int pl_channel_diagnostics(pl_channel *c, pl_diag *out)
 {
-    if (launch_diagnostics_fp64(c->u, c->v, c->w, c->sp, c->m, c->d_diag, c->d_loc, c->d_dpart, c->d_dipart,
-                                c->max_blocks, c->stream))
+    int *d_loc = reinterpret_cast<int *>(c->d_diag + 4);
+    if (launch_diagnostics_fp64(c->u, c->v, c->w, c->sp, c->m, c->d_diag, d_loc, c->d_dpart, c->d_dipart, c->max_blocks,
+                                c->stream))
         return -1;
-    double h[3];
-    int loc[6];
+    double h[8];
     PL_CUDA_TRY(cudaMemcpyAsync(h, c->d_diag, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    PL_CUDA_TRY(cudaMemcpyAsync(loc, c->d_loc, sizeof(loc), cudaMemcpyDeviceToHost, c->stream));
     PL_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    int loc[6];
+    std::memcpy(loc, h + 4, sizeof(loc));
     out->div_max = h[0];
     out->cfl_max = h[1];
     out->nan_count = (int)h[2];

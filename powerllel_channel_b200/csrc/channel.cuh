@@ -46,8 +46,11 @@ struct pl_channel {
     pl::Ppe ppe;
     pl::ReduceBuf rb;
     pl::MeanState ms;
-    double *d_diag = nullptr;
-    int *d_loc = nullptr;
+    double *d_diag = nullptr; // [0..3] values, [4..] the locations (int)
+    // the monitors' and the kinetic energy's scratch: results, then partial sums
+    double *d_mon = nullptr;
+    unsigned int *d_mon_count = nullptr; // zero between launches
+    void *adj = nullptr;                 // the adjoint's fields and checkpoints (adjoint.cu), once used
     double *d_dpart = nullptr;
     long long *d_dipart = nullptr;
     int max_blocks = 0;
@@ -58,7 +61,11 @@ struct pl_channel {
     std::vector<std::string> *prof_names = nullptr;
 };
 
+// d_mon: MON_OUT results, then partial sums: MON_PARTS per plane and component
+constexpr int MON_OUT = 8, MON_PARTS = 8;
+
 namespace pl {
+void adjoint_free(pl_channel *c);
 // the FP64 pressure of the current state (the mixed path widens p32 into p
 // on the channel's stream when it has changed)
 const double *channel_p64(pl_channel *c);

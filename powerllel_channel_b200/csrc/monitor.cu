@@ -49,51 +49,55 @@ __global__ void __launch_bounds__(256) k_stat_sample(const double *__restrict__ 
         if (s.a[q]) s.a[q][o] += val[q];
 }
 
-// deterministic sums over the (i, j) plane k of var (ghosted velocity layout):
-// part[b] for each of `nb` blocks, then k_sum_finish adds them in order
-__global__ void __launch_bounds__(256) k_plane_part(const double *__restrict__ var, int k, StepParams p,
-                                                    double *__restrict__ part)
+// sum over the planes k0 .. k0 + gridDim.y - 1 of var (ghosted velocity
+// layout), each plane's sum times weight[k] where weights are given.  A plane
+// is split over gridDim.x blocks; the last block to finish adds the partials
+// up as a tree, in an order fixed by their positions.  One launch: as a
+// partial-sum kernel and a one-thread loop over its output, Mean_h of a
+// 256x192x128 field took 128 CTAs for the planes and 128 dependent loads.
+__global__ void __launch_bounds__(256) k_planes_sum(const double *__restrict__ var, int k0, const double *weight,
+                                                    StepParams p, double *part, unsigned int *counter, double *out)
 {
     __shared__ double sh[256];
+    __shared__ bool last;
+    const int t = threadIdx.x, k = k0 + blockIdx.y, nb = gridDim.x * gridDim.y;
     const size_t sk = (size_t)p.nx * p.ny;
-    double s = 0.0;
-    for (size_t q = (size_t)blockIdx.x * 256 + threadIdx.x; q < sk; q += (size_t)gridDim.x * 256)
-        s += __ldg(var + sk * k + q);
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-        if (threadIdx.x < h) sh[threadIdx.x] += sh[threadIdx.x + h];
+    auto tree = [&](double s) {
+        sh[t] = s;
         __syncthreads();
+        for (int h = 128; h > 0; h >>= 1) {
+            if (t < h) sh[t] += sh[t + h];
+            __syncthreads();
+        }
+    };
+    double s = 0.0;
+    for (size_t q = (size_t)blockIdx.x * 256 + t; q < sk; q += (size_t)gridDim.x * 256) s += __ldg(var + sk * k + q);
+    tree(s);
+    if (t == 0) {
+        part[blockIdx.x + gridDim.x * blockIdx.y] = weight ? sh[0] * __ldg(weight + k) : sh[0];
+        __threadfence();
+        last = atomicAdd(counter, 1u) == (unsigned)nb - 1;
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    s = 0.0;
+    for (int q = t; q < nb; q += 256) s += __ldcg(part + q);
+    tree(s);
+    if (t == 0) {
+        *out = sh[0];
+        *counter = 0u;
+    }
 }
 
-// Mean_h (mod_utils.f90:105-131): sum of var * dzf/lz over the interior / (nx ny);
-// per-level partials in k order
-__global__ void __launch_bounds__(256) k_meanh_part(const double *__restrict__ var, StepParams p, MeshDev m,
-                                                    double *__restrict__ part)
+// u, v, w (at g) and p (at o) of one point, side by side for one copy
+__global__ void k_probe(const double *u, const double *v, const double *w, const double *pp, size_t g, size_t o,
+                        double *out)
 {
-    __shared__ double sh[256];
-    const int k = blockIdx.x + 1;
-    const size_t sk = (size_t)p.nx * p.ny;
-    double s = 0.0;
-    for (size_t q = threadIdx.x; q < sk; q += 256) s += __ldg(var + sk * k + q);
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-        if (threadIdx.x < h) sh[threadIdx.x] += sh[threadIdx.x + h];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0] * __ldg(m.dzflzi + k);
-}
-
-__global__ void k_sum_finish(const double *__restrict__ part, int n, double *__restrict__ out)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int q = 0; q < n; q++) s += part[q];
-        *out = s;
-    }
+    out[0] = u[g];
+    out[1] = v[g];
+    out[2] = w[g];
+    out[3] = pp[o];
 }
 
 // extractRegion (mod_monitor.f90:323-376): cell-centred u, v, w (+u_crf on u)
@@ -248,15 +252,10 @@ extern "C" int pl_monitor_skin_friction(pl_channel *c, int wall, double *u_tau, 
     // calcAndWriteSkf (:264-296): tau_w = mean of re_inv (u(k_wall) + u_crf) / dz,
     // dz = dzf(k_wall)/2, k_wall = 1 or nz
     const int kw = wall == 0 ? 1 : c->nz;
-    constexpr int NB = 64;
-    double *part = nullptr;
-    PL_CUDA_TRY(cudaMalloc(&part, sizeof(double) * (NB + 1)));
-    k_plane_part<<<NB, 256, 0, c->stream>>>(c->u, kw, c->sp, part);
-    k_sum_finish<<<1, 32, 0, c->stream>>>(part, NB, part + NB);
     double sum = 0.0;
-    int rc = (cudaGetLastError() == cudaSuccess) ? host_scalar(c, part + NB, &sum) : -1;
-    cudaFree(part);
-    if (rc) {
+    k_planes_sum<<<dim3(64, 1), 256, 0, c->stream>>>(c->u, kw, nullptr, c->sp, c->d_mon + MON_OUT, c->d_mon_count,
+                                                     c->d_mon);
+    if (cudaGetLastError() != cudaSuccess || host_scalar(c, c->d_mon, &sum)) {
         set_error("pl_monitor_skin_friction: device error");
         return -1;
     }
@@ -272,23 +271,18 @@ extern "C" int pl_monitor_skin_friction(pl_channel *c, int wall, double *u_tau, 
 extern "C" int pl_monitor_forcing(pl_channel *c, double vel_mean[3])
 {
     // calcAndWriteForcing (:298-318): Mean_h of the forced components, u_crf added to u
-    double *part = nullptr;
-    PL_CUDA_TRY(cudaMalloc(&part, sizeof(double) * ((size_t)c->nz + 1)));
     const double *f[3] = {c->u, c->v, c->w};
-    int rc = 0;
-    for (int d = 0; d < 3 && rc == 0; d++) {
+    for (int d = 0; d < 3; d++) {
         vel_mean[d] = 0.0;
         if (!c->cfg.is_forced[d]) continue;
-        k_meanh_part<<<c->nz, 256, 0, c->stream>>>(f[d], c->sp, c->m, part);
-        k_sum_finish<<<1, 32, 0, c->stream>>>(part, c->nz, part + c->nz);
+        k_planes_sum<<<dim3(MON_PARTS, c->nz), 256, 0, c->stream>>>(f[d], 1, c->m.dzflzi, c->sp, c->d_mon + MON_OUT,
+                                                                    c->d_mon_count, c->d_mon);
         double s = 0.0;
-        rc = (cudaGetLastError() == cudaSuccess) ? host_scalar(c, part + c->nz, &s) : -1;
+        if (cudaGetLastError() != cudaSuccess || host_scalar(c, c->d_mon, &s)) {
+            set_error("pl_monitor_forcing: device error");
+            return -1;
+        }
         vel_mean[d] = s / c->nx / c->ny;
-    }
-    cudaFree(part);
-    if (rc) {
-        set_error("pl_monitor_forcing: device error");
-        return -1;
     }
     vel_mean[0] += c->cfg.u_crf;
     return 0;
@@ -303,9 +297,9 @@ extern "C" int pl_monitor_probe(pl_channel *c, int i, int j, int k, double out[4
     }
     const size_t sk = (size_t)c->nx * c->ny;
     const size_t g = (size_t)(i - 1) + (size_t)c->nx * (j - 1) + sk * k;
-    const double *src[4] = {c->u + g, c->v + g, c->w + g, state_p(c) + g - sk};
-    for (int q = 0; q < 4; q++)
-        PL_CUDA_TRY(cudaMemcpyAsync(out + q, src[q], sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    k_probe<<<1, 1, 0, c->stream>>>(c->u, c->v, c->w, state_p(c), g, g - sk, c->d_mon);
+    PL_CHECK_LAUNCH();
+    PL_CUDA_TRY(cudaMemcpyAsync(out, c->d_mon, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     PL_CUDA_TRY(cudaStreamSynchronize(c->stream));
     out[0] += c->cfg.u_crf;
     return 0;

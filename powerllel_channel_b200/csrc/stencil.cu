@@ -182,32 +182,45 @@ __device__ __forceinline__ void better(double &v, long long &ix, double ov, long
     }
 }
 
+// A block takes 64 x 4 points of DIAG_PLANES planes, so that the partials left
+// to the second kernel are few and each thread has several loads in flight.
+constexpr int DIAG_PLANES = 8;
+static inline dim3 diag_grid(const StepParams &p)
+{
+    return dim3((p.nx + 63) / 64, (p.ny + 3) / 4, (p.nz + DIAG_PLANES - 1) / DIAG_PLANES);
+}
 __global__ void __launch_bounds__(256) k_diag(const double *__restrict__ u, const double *__restrict__ v,
                                               const double *__restrict__ w, StepParams p, MeshDev m,
                                               double *part, long long *ipart)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z + 1;
     double dv = -1.0, cv = -1.0, nan = 0.0;
     long long di = 0x7fffffffffffffffLL, ci = 0x7fffffffffffffffLL;
     if (i < p.nx && j < p.ny) {
-        const Nb n = neighbours(i, j, k, p.nx, p.ny);
-        const double dzfi = __ldg(m.dzf_inv + k);
-        const double uc = __ldg(u + n.c), vc = __ldg(v + n.c), wc = __ldg(w + n.c);
-        const double um = __ldg(u + n.xm), vm = __ldg(v + n.ym), wm = __ldg(w + n.zm);
-        dv = fabs((uc - um) * p.dx_inv + (vc - vm) * p.dy_inv + (wc - wm) * dzfi);
-        cv = fabs((uc + um) * 0.5) * p.dx_inv + fabs((vc + vm) * 0.5) * p.dy_inv + fabs((wc + wm) * 0.5) * dzfi;
-        const long long lin = (long long)i + (long long)p.nx * (j + (long long)p.ny * (k - 1));
-        di = ci = lin;
-        nan = (uc != uc) + (vc != vc) + (wc != wc);
-        if (k == 1) nan += (__ldg(u + n.zm) != __ldg(u + n.zm)) + (vm != vm) + (wm != wm);
-        if (k == p.nz)
-            nan += (__ldg(u + n.zp) != __ldg(u + n.zp)) + (__ldg(v + n.zp) != __ldg(v + n.zp)) +
-                   (__ldg(w + n.zp) != __ldg(w + n.zp));
-        // NaN compares false: map a NaN residual to +inf so it is reported
-        if (dv != dv) dv = __longlong_as_double(0x7ff0000000000000LL);
-        if (cv != cv) cv = __longlong_as_double(0x7ff0000000000000LL);
+        const int k0 = blockIdx.z * DIAG_PLANES + 1;
+#pragma unroll
+        for (int q = 0; q < DIAG_PLANES; q++) {
+            const int k = k0 + q;
+            if (k > p.nz) break;
+            const Nb n = neighbours(i, j, k, p.nx, p.ny);
+            const double dzfi = __ldg(m.dzf_inv + k);
+            const double uc = __ldg(u + n.c), vc = __ldg(v + n.c), wc = __ldg(w + n.c);
+            const double um = __ldg(u + n.xm), vm = __ldg(v + n.ym), wm = __ldg(w + n.zm);
+            double d = fabs((uc - um) * p.dx_inv + (vc - vm) * p.dy_inv + (wc - wm) * dzfi);
+            double c = fabs((uc + um) * 0.5) * p.dx_inv + fabs((vc + vm) * 0.5) * p.dy_inv + fabs((wc + wm) * 0.5) * dzfi;
+            const long long lin = (long long)i + (long long)p.nx * (j + (long long)p.ny * (k - 1));
+            nan += (uc != uc) + (vc != vc) + (wc != wc);
+            if (k == 1) nan += (__ldg(u + n.zm) != __ldg(u + n.zm)) + (vm != vm) + (wm != wm);
+            if (k == p.nz)
+                nan += (__ldg(u + n.zp) != __ldg(u + n.zp)) + (__ldg(v + n.zp) != __ldg(v + n.zp)) +
+                       (__ldg(w + n.zp) != __ldg(w + n.zp));
+            // NaN compares false: map a NaN residual to +inf so it is reported
+            if (d != d) d = __longlong_as_double(0x7ff0000000000000LL);
+            if (c != c) c = __longlong_as_double(0x7ff0000000000000LL);
+            better(dv, di, d, lin);
+            better(cv, ci, c, lin);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         double odv = __shfl_down_sync(0xffffffffu, dv, o), ocv = __shfl_down_sync(0xffffffffu, cv, o);
@@ -668,9 +681,10 @@ int launch_diagnostics_fp64(const double *u, const double *v, const double *w, c
         set_error("diagnostics buffer too small");
         return -1;
     }
-    k_diag<<<point_grid(p), point_block(), 0, st>>>(u, v, w, p, m, d_part, d_ipart);
+    const dim3 g = diag_grid(p);
+    k_diag<<<g, point_block(), 0, st>>>(u, v, w, p, m, d_part, d_ipart);
     PL_CHECK_LAUNCH();
-    k_diag_finish<<<1, DIAG_FIN_THREADS, 0, st>>>(d_part, d_ipart, nblocks(p), p, d_out, d_loc);
+    k_diag_finish<<<1, DIAG_FIN_THREADS, 0, st>>>(d_part, d_ipart, (int)(g.x * g.y * g.z), p, d_out, d_loc);
     PL_CHECK_LAUNCH();
     return 0;
 }
