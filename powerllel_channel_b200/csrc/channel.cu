@@ -252,7 +252,6 @@ static void channel_free(pl_channel *c)
     cudaFree(c->p32);
     cudaFree(c->pm32);
     cudaFree(c->pb32);
-    if (c->mxtab) cudaFree(c->mxtab - (size_t)12 * c->hx);
     cudaFree(c->d1u);
     cudaFree(c->d1v);
     cudaFree(c->d1w);
@@ -371,10 +370,7 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
         cudaMemset(*f, 0, sizeof(float) * n);
         return true;
     };
-    // both RK stages in one kernel: FP64 on every grid, mixed where the grid
-    // tiles by 32 x 16; else the two stage kernels
-    c->fused_rk = !mixed || rk_mixed_supported(c->sp);
-    if (zn > 1 && !(mixed ? c->fused_rk : c->nx % 32 == 0 && c->ny % 8 == 0)) {
+    if (zn > 1 && (c->nx % 32 != 0 || c->ny % (mixed ? 16 : 8) != 0)) {
         set_error("pl_channel_create_slab: the slab step needs the fused RK kernel: nx % 32 == 0 and ny % 8 == 0 "
                   "(FP64) or ny % 16 == 0 (mixed)");
         return fail();
@@ -392,9 +388,8 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
     if (ok && !mixed && zn == 1) ok = valloc(&c->u1) && valloc(&c->v1) && valloc(&c->w1);
     if (ok && mixed) {
         ok = falloc(&c->p32, c->np) && falloc(&c->pb32, c->np) && falloc(&c->pm32, c->np) &&
-             falloc(&c->mxtab, (size_t)12 * n1) && falloc(&c->r32, npx) && dalloc(&c->mode0, c->nz) &&
+             falloc(&c->r32, npx) && dalloc(&c->mode0, c->nz) &&
              dalloc(&c->plane_part, (size_t)std::max(warp_partials_per_plane(c->sp), c->sp.ny / 2) * c->nz);
-        if (ok) c->mxtab += (size_t)12 * hx;
         if (ok && zn == 1) ok = falloc(&c->d1u, c->nf) && falloc(&c->d1v, c->nf) && falloc(&c->d1w, c->nf);
     }
     if (!ok) {
@@ -409,17 +404,8 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
     if (zn > 1 ? ppe_create_slab(&c->ppe, c->nx, c->ny, cfg->nz, dx, dy, c->dzf_global.data(), zn, c->zrank, pprec)
                : ppe_create(&c->ppe, c->nx, c->ny, c->nz, dx, dy, c->dzf_global.data(), cfg->trid_parts, pprec))
         return fail();
-    if (mixed) {
-        const std::vector<float> tab = rk_mixed_table(c->sp, c->dzf, c->dzf_inv, c->dzc_inv, kst - hx, n1);
-        if (cudaMemcpy(c->mxtab - (size_t)12 * hx, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice) !=
-            cudaSuccess) {
-            set_error("pl_channel_create: upload of the mixed RK coefficients failed");
-            return fail();
-        }
-    }
     c->max_blocks = ((c->nx + 63) / 64) * ((c->ny + 3) / 4) * c->nz;
-    if (!mixed && rk_fused_blocks(c->sp) > c->max_blocks) c->max_blocks = rk_fused_blocks(c->sp);
-    if (c->fused_rk && mixed && rk_mixed_blocks(c->sp) > c->max_blocks) c->max_blocks = rk_mixed_blocks(c->sp);
+    c->max_blocks = std::max(c->max_blocks, mixed ? rk_mixed_blocks(c->sp) : rk_fused_blocks(c->sp));
     c->rb.max_blocks = c->max_blocks;
     if (cudaMalloc(&c->rb.partial, sizeof(double) * 3 * c->max_blocks) != cudaSuccess ||
         cudaMalloc(&c->rb.scalar, sizeof(double) * 8) != cudaSuccess ||
@@ -641,19 +627,12 @@ extern "C" int pl_phase_correct_force(pl_channel *c)
     return rc;
 }
 
-// both RK stages in one kernel (out of place; mixed: when the grid tiles by
-// 32 x 16), else the two stage kernels
+// both RK stages in one kernel (out of place)
 extern "C" int pl_phase_rk(pl_channel *c)
 {
-    int rc;
-    if (!c->fused_rk) {
-        rc = pl_phase_rk1(c);
-        if (!rc) rc = pl_phase_rk2(c);
-        return rc;
-    }
-    rc = is_mixed(c) ? launch_rk_mixed(c->u, c->v, c->w, c->ub, c->vb, c->wb, c->sp, c->m, c->mxtab, c->ms, c->pm32,
-                                       mixed_incremental(c), c->stream)
-                     : launch_rk_fused_fp64(c->u, c->v, c->w, c->ub, c->vb, c->wb, c->sp, c->m, c->ms, c->stream);
+    const int rc = is_mixed(c) ? launch_rk_mixed(c->u, c->v, c->w, c->ub, c->vb, c->wb, c->sp, c->m, c->ms, c->pm32,
+                                                 mixed_incremental(c), c->stream)
+                               : launch_rk_fused_fp64(c->u, c->v, c->w, c->ub, c->vb, c->wb, c->sp, c->m, c->ms, c->stream);
     std::swap(c->u, c->ub);
     std::swap(c->v, c->vb);
     std::swap(c->w, c->wb);
@@ -918,14 +897,7 @@ extern "C" int pl_slab_init_finish(pl_channel *c)
     return rc;
 }
 
-extern "C" int pl_slab_rk(pl_channel *c)
-{
-    if (!c->fused_rk) {
-        set_error("pl_slab_rk: the slab step needs the fused RK kernel");
-        return -1;
-    }
-    return pl_phase_rk(c);
-}
+extern "C" int pl_slab_rk(pl_channel *c) { return pl_phase_rk(c); }
 
 extern "C" int pl_slab_mean_finish(pl_channel *c)
 {

@@ -30,19 +30,17 @@ struct pl_channel {
     // (FP32, updated in place by the solve); the pressure prediction for the
     // next projection in pm32, written into pb32 by the solve and swapped;
     // the PPE works in place on r32 (FP32); p (FP64) is p32 widened on demand
-    // for readers (channel_p64); mxtab: the mixed RK kernel's per-plane
-    // coefficients
+    // for readers (channel_p64)
     double *u = nullptr, *v = nullptr, *w = nullptr;
     double *u1 = nullptr, *v1 = nullptr, *w1 = nullptr;
     double *p = nullptr;
     double *ub = nullptr, *vb = nullptr, *wb = nullptr;
-    float *p32 = nullptr, *pm32 = nullptr, *pb32 = nullptr, *mxtab = nullptr;
+    float *p32 = nullptr, *pm32 = nullptr, *pb32 = nullptr;
     bool p_stale = false; // mixed: p lags p32
     float *d1u = nullptr, *d1v = nullptr, *d1w = nullptr, *r32 = nullptr;
     double *plane_part = nullptr, *mode0 = nullptr;
     int incremental = 1;   // mixed path: solve for a pressure increment (Thomas)
     long long nsolve = 0;  // projections since the initial field (mixed prediction schedule)
-    bool fused_rk = false; // both RK stages in one kernel (rk_fused.cu, rk_mixed.cu)
     pl::Ppe ppe;
     pl::ReduceBuf rb;
     pl::MeanState ms;

@@ -421,14 +421,12 @@ static dim3 fused_tiles(const StepParams &p) { return dim3((p.nx + FX - 1) / FX,
 // Planes per z-chunk: the count of waves of resident CTAs times a chunk's
 // planes plus the few it recomputes or waits for, whichever chunk count gives
 // least (a grid that does not fill the chip takes short chunks).
-static int fused_kchunk(const StepParams &p, int resident)
+int rk_kchunk(long tiles, int nz, int most, int resident)
 {
-    const dim3 t = fused_tiles(p);
-    const long tiles = (long)t.x * t.y;
     int best = 0;
     long cost = 0;
-    for (int kc = min(p.nz, F_KCHUNK); kc >= 2; kc--) {
-        const long ctas = tiles * ((p.nz + kc - 1) / kc);
+    for (int kc = min(nz, most); kc >= 2; kc--) {
+        const long ctas = tiles * ((nz + kc - 1) / kc);
         const long c = ((ctas + resident - 1) / resident) * (kc + 5);
         if (best == 0 || c < cost) {
             best = kc;
@@ -459,8 +457,8 @@ int launch_rk_fused_fp64(const double *u, const double *v, const double *w, doub
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FT, shm) != cudaSuccess || per_sm < 1) per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int kchunk = fused_kchunk(p, per_sm * (nsm > 0 ? nsm : 1));
     dim3 grid = fused_tiles(p);
+    const int kchunk = rk_kchunk((long)grid.x * grid.y, p.nz, F_KCHUNK, per_sm * (nsm > 0 ? nsm : 1));
     grid.z = (p.nz + kchunk - 1) / kchunk;
     if ((int)(grid.x * grid.y * grid.z) > ms.max_blocks) {
         set_error("mean buffer too small for the fused RK kernel");

@@ -3,8 +3,6 @@
 // src/mod_calcRHS.f90, src/mod_updateBound.f90, src/mod_utils.f90).
 #pragma once
 
-#include <vector>
-
 #include "common.cuh"
 
 namespace pl {
@@ -63,27 +61,13 @@ int launch_rk_fused_fp64(const double *u, const double *v, const double *w, doub
 
 // mixed path: both RK stages in FP32 flux form (rk_mixed.cu); with pinc,
 // u_hat = u* - dt G pq is stored (pq: the FP32 pressure prediction,
-// interior-only layout), whose divergence / dt is the increment's residual.
-// tab: the per-plane coefficients of rk_mixed_table, 12 floats per plane
-// k = 0..nz+1, on the device.
-struct MxPlane {
-    float a, b;                 // face weights: q_{k+1/2} = q_k a + q_{k+1} b
-    float hzuv, azp, azm, ccuv; // u, v equations (dt folded in)
-    float hzw, bzp, bzm, ccw;   // w equation
-    float gz;                   // dt dzc_inv(k)
-};
-struct MxConst {
-    float hx, hy, cxx, cyy, ucx, gx, gy;
-};
-bool rk_mixed_supported(const StepParams &p);
+// interior-only layout), whose divergence / dt is the increment's residual
 int rk_mixed_blocks(const StepParams &p);
-// the table's np planes from global plane kg0 on (the mesh vectors are global)
-std::vector<float> rk_mixed_table(const StepParams &p, const std::vector<double> &dzf,
-                                  const std::vector<double> &dzf_inv, const std::vector<double> &dzc_inv, int kg0,
-                                  size_t np);
 int launch_rk_mixed(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
-                    const StepParams &p, const MeshDev &m, const float *tab, MeanState &ms, const float *pq, int pinc,
-                    cudaStream_t st);
+                    const StepParams &p, const MeshDev &m, MeanState &ms, const float *pq, int pinc, cudaStream_t st);
+// planes per z-chunk of the fused RK kernels (at most `most`) for a grid of
+// `tiles` tile columns, `resident` CTAs fitting the chip at once
+int rk_kchunk(long tiles, int nz, int most, int resident);
 
 int launch_rk2m_fp64(double *u, double *v, double *w, const double *u1, const double *v1, const double *w1,
                      const StepParams &p, const MeshDev &m, MeanState &ms, cudaStream_t st);
