@@ -405,6 +405,7 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
                : ppe_create(&c->ppe, c->nx, c->ny, c->nz, dx, dy, c->dzf_global.data(), cfg->trid_parts, pprec))
         return fail();
     c->max_blocks = ((c->nx + 63) / 64) * ((c->ny + 3) / 4) * c->nz;
+    if (mixed ? rk_mixed_prepare(c->sp, &c->rk) : rk_fused_prepare(c->sp, &c->rk)) return fail();
     c->max_blocks = std::max(c->max_blocks, mixed ? rk_mixed_blocks(c->sp) : rk_fused_blocks(c->sp));
     c->rb.max_blocks = c->max_blocks;
     if (cudaMalloc(&c->rb.partial, sizeof(double) * 3 * c->max_blocks) != cudaSuccess ||
@@ -583,14 +584,7 @@ extern "C" int pl_phase_poisson(pl_channel *c)
 // plane sums are summed per line pair instead of per warp.
 static int phase_rhs_poisson(pl_channel *c)
 {
-    DivIn d;
-    d.u = c->u;
-    d.v = c->v;
-    d.w = c->w;
-    d.dzf_inv = c->m.dzf_inv;
-    d.dti = 1.0 / c->sp.dt;
-    d.dtidxi = d.dti * c->sp.dx_inv;
-    d.dtidyi = d.dti * c->sp.dy_inv;
+    const DivIn d = channel_div_in(c, c->u, c->v, c->w);
     if (is_mixed(c)) {
         const int rc = ppe_xfwd_div<float>(&c->ppe, d, c->r32, c->plane_part, c->stream);
         if (rc < 0) return -1;
@@ -631,8 +625,9 @@ extern "C" int pl_phase_correct_force(pl_channel *c)
 extern "C" int pl_phase_rk(pl_channel *c)
 {
     const int rc = is_mixed(c) ? launch_rk_mixed(c->u, c->v, c->w, c->ub, c->vb, c->wb, c->sp, c->m, c->ms, c->pm32,
-                                                 mixed_incremental(c), c->stream)
-                               : launch_rk_fused_fp64(c->u, c->v, c->w, c->ub, c->vb, c->wb, c->sp, c->m, c->ms, c->stream);
+                                                 mixed_incremental(c), c->rk, c->stream)
+                               : launch_rk_fused_fp64(c->u, c->v, c->w, c->ub, c->vb, c->wb, c->sp, c->m, c->ms, c->rk,
+                                                      c->stream);
     std::swap(c->u, c->ub);
     std::swap(c->v, c->vb);
     std::swap(c->w, c->wb);
@@ -907,14 +902,7 @@ extern "C" int pl_slab_mean_finish(pl_channel *c)
 // calcRHS fused into the forward x transform, the y transform, the local PDD sweep
 extern "C" int pl_slab_rhs_sweep(pl_channel *c)
 {
-    DivIn d;
-    d.u = c->u;
-    d.v = c->v;
-    d.w = c->w;
-    d.dzf_inv = c->m.dzf_inv;
-    d.dti = 1.0 / c->sp.dt;
-    d.dtidxi = d.dti * c->sp.dx_inv;
-    d.dtidyi = d.dti * c->sp.dy_inv;
+    const DivIn d = channel_div_in(c, c->u, c->v, c->w);
     int rc = is_mixed(c) ? ppe_xfwd_div<float>(&c->ppe, d, c->r32, c->plane_part, c->stream)
                          : ppe_xfwd_div<double>(&c->ppe, d, c->p, nullptr, c->stream);
     if (rc < 0) return -1;

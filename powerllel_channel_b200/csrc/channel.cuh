@@ -44,6 +44,7 @@ struct pl_channel {
     pl::Ppe ppe;
     pl::ReduceBuf rb;
     pl::MeanState ms;
+    pl::RkLaunch rk;
     double *d_diag = nullptr; // [0..3] values, [4..] the locations (int)
     // the monitors' and the kinetic energy's scratch: results, then partial sums
     double *d_mon = nullptr;
@@ -63,6 +64,19 @@ struct pl_channel {
 constexpr int MON_OUT = 8, MON_PARTS = 8;
 
 namespace pl {
+// the operands of calcRHS fused into the forward x transform, for these fields
+inline DivIn channel_div_in(const pl_channel *c, const double *u, const double *v, const double *w)
+{
+    DivIn d;
+    d.u = u;
+    d.v = v;
+    d.w = w;
+    d.dzf_inv = c->m.dzf_inv;
+    d.dti = 1.0 / c->sp.dt;
+    d.dtidxi = d.dti * c->sp.dx_inv;
+    d.dtidyi = d.dti * c->sp.dy_inv;
+    return d;
+}
 void adjoint_free(pl_channel *c);
 // the FP64 pressure of the current state (the mixed path widens p32 into p
 // on the channel's stream when it has changed)

@@ -44,6 +44,36 @@ const char *get_error();
         }                                                                                  \
     } while (0)
 
+// Launch of a kernel that begins with pdl_enter(): its CTAs may be scheduled
+// while the stream's previous kernel drains, and wait there for its results.
+// The step is a chain of eight short kernels, whose launch latencies add up on
+// small grids.
+template <typename... K, typename... A>
+inline cudaError_t launch_chained(void (*kern)(K...), dim3 grid, dim3 block, size_t shm, cudaStream_t st, A &&...args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = shm;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<K>(args)...);
+}
+
+// First statement of such a kernel: waits until the previous kernel of the
+// stream has completed and its writes are visible (it waited for its own
+// predecessor in turn), then lets the next one's CTAs be scheduled.  Without
+// the launch attribute both are no-ops.
+__device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 template <typename T> struct cplx_of;
 template <> struct cplx_of<double> { using type = double2; };
 template <> struct cplx_of<float> { using type = float2; };

@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(256) k_xfft_ct(const T *__restrict__ in, size_
                                                  T *__restrict__ out, size_t out_off, size_t out_sj, size_t out_sk,
                                                  const typename cplx_of<T>::type *__restrict__ twg, int ny, T scale)
 {
+    pdl_enter();
     using V = typename cplx_of<T>::type;
     constexpr int NB = ct_x_lines<N>(), BUF = fpad_elems<V>(NB * N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -146,6 +147,7 @@ __global__ void __launch_bounds__(pf_x_threads<T>()) k_xfft_pf(const T *__restri
                                                                const typename cplx_of<T>::type *__restrict__ twg,
                                                                int ny, int total, T scale, PressureUpdate pu)
 {
+    pdl_enter();
     static_assert(!PU || (sizeof(T) == 4 && !FWD), "the fused pressure update is the FP32 inverse's");
     using V = typename cplx_of<T>::type;
     constexpr int NT = pf_x_threads<T>();
@@ -252,6 +254,7 @@ __global__ void __launch_bounds__(pf_y_threads<T>(),
     k_yfft_pf(T *__restrict__ data, const typename cplx_of<T>::type *__restrict__ twg,
                                                  int nx, int total)
 {
+    pdl_enter();
     using V = typename cplx_of<T>::type;
     constexpr int NT = pf_y_threads<T>();
     constexpr int W = pf_y_cols<V, N, FWD>(), BUF = (fpad_elems<V>(W * N) + 1) / 2 * 2, RAW = W * N;
@@ -331,8 +334,8 @@ template <typename T, int N> __host__ __device__ constexpr int xdiv_smem_bytes()
 {
     using V = typename cplx_of<T>::type;
     constexpr int NB = xdiv_lines(N);
-    // work buffer, 8 NB + 1 staged FP64 rows, per-stage twiddles, 2 warp sums
-    return (int)(sizeof(V) * ((fpad_elems<V>(NB * N) + 1) / 2 * 2) + 8 * (8 * NB + 1) * N + sizeof(V) * N + 16);
+    // work buffer, 8 NB + 1 staged FP64 rows, per-stage twiddles, warp sums
+    return (int)(sizeof(V) * ((fpad_elems<V>(NB * N) + 1) / 2 * 2) + 8 * (8 * NB + 1) * N + sizeof(V) * N + 32);
 }
 
 template <typename T, int N>
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(XDIV_THREADS) k_xfft_div_pf(DivIn d, T *__rest
                                                               const typename cplx_of<T>::type *__restrict__ twg,
                                                               int ny, int total, double *__restrict__ part)
 {
+    pdl_enter();
     using V = typename cplx_of<T>::type;
     constexpr int NT = XDIV_THREADS, NB = xdiv_lines(N), BUF = (fpad_elems<V>(NB * N) + 1) / 2 * 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -391,7 +395,8 @@ __global__ void __launch_bounds__(XDIV_THREADS) k_xfft_div_pf(DivIn d, T *__rest
             if ((tid & 31) == 0) wsum[tid >> 5] = acc;
         }
         __syncthreads();
-        if (part != nullptr && tid == 0) part[g] = wsum[0] + wsum[1];
+        if (part != nullptr && tid == 0)
+            part[g] = NT == 64 ? wsum[0] + wsum[1] : (wsum[0] + wsum[1]) + (wsum[2] + wsum[3]);
         if (g + (int)gridDim.x < total) fetch(g + gridDim.x);
         T *dst = out + (size_t)k * N * ny + (size_t)2 * p * N;
         ct_batch_ip<V, true, false, N, NB, 1, N, NT, 1, ct_nstages(N) - 1>(buf, nb, tw, tid);
@@ -405,81 +410,120 @@ __global__ void __launch_bounds__(XDIV_THREADS) k_xfft_div_pf(DivIn d, T *__rest
     cp_async_wait<0>();
 }
 
-template <typename T, int N, bool FWD>
-int launch_x_ct(const Ppe *s, const T *in, size_t in_off, size_t in_sj, size_t in_sk, T *out, size_t out_off,
-                       size_t out_sj, size_t out_sk, T scale, cudaStream_t st, const PressureUpdate *pu, bool *fused)
+// shared memory (bytes) of the kernels of a length
+template <typename T, int N> constexpr size_t x_pf_bytes() { return sizeof(typename cplx_of<T>::type) * (size_t)pf_x_smem_elems<T, N>(); }
+template <typename T, int N> constexpr size_t x_ct_bytes()
 {
     using V = typename cplx_of<T>::type;
-    constexpr int NB = ct_x_lines<N>();
-    const size_t shm = sizeof(V) * (2 * (size_t)fpad_elems<V>(NB * N) + N);
+    return sizeof(V) * (2 * (size_t)fpad_elems<V>(ct_x_lines<N>() * N) + N);
+}
+template <typename T, int N, bool FWD> constexpr size_t y_pf_bytes()
+{
+    return sizeof(typename cplx_of<T>::type) * (size_t)pf_y_smem_elems<T, N, FWD>();
+}
+template <typename T, int N> int x_pf_groups(const Ppe *s) { return ((s->ny / 2 + pf_x_lines<T, N>() - 1) / pf_x_lines<T, N>()) * s->nz; }
+template <typename T, int N, bool FWD> int y_pf_groups(const Ppe *s)
+{
+    constexpr int W = pf_y_cols<typename cplx_of<T>::type, N, FWD>();
+    return ((s->nx / 2 + W - 1) / W) * s->nz;
+}
+template <int N> int xdiv_groups(const Ppe *s) { return ((s->ny / 2 + xdiv_lines(N) - 1) / xdiv_lines(N)) * s->nz; }
+
+// the kernel's shared-memory limit and its grid: all groups, or what the chip holds at once
+template <typename K> int persistent_grid(K kernel, size_t shm, int total, int threads, int *grid)
+{
+    if (shm > 48 * 1024)
+        PL_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, shm) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    *grid = std::max(1, std::min(total, per_sm * sm_count()));
+    return 0;
+}
+
+template <typename T, int N> int prepare_x_ct(Ppe *s)
+{
+    constexpr int NT = pf_x_threads<T>();
+    const int groups = x_pf_groups<T, N>(s);
+    if (x_ct_bytes<T, N>() > 48 * 1024) {
+        PL_CUDA_TRY(cudaFuncSetAttribute(k_xfft_ct<T, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)x_ct_bytes<T, N>()));
+        PL_CUDA_TRY(cudaFuncSetAttribute(k_xfft_ct<T, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)x_ct_bytes<T, N>()));
+    }
+    if (persistent_grid(k_xfft_pf<T, N, true>, x_pf_bytes<T, N>(), groups, NT, &s->grid_x[0]) ||
+        persistent_grid(k_xfft_pf<T, N, false>, x_pf_bytes<T, N>(), groups, NT, &s->grid_x[1]) ||
+        persistent_grid(k_xfft_div_pf<T, N>, xdiv_smem_bytes<T, N>(), xdiv_groups<N>(s), XDIV_THREADS, &s->grid_x[3]))
+        return -1;
+    if constexpr (sizeof(T) == 4)
+        return persistent_grid(k_xfft_pf<T, N, false, true>, x_pf_bytes<T, N>() + pf_x_pu_bytes<T, N>(), groups, NT,
+                               &s->grid_x[2]);
+    return 0;
+}
+
+template <typename T, int N> int prepare_y_ct(Ppe *s)
+{
+    constexpr int NT = pf_y_threads<T>();
+    return persistent_grid(k_yfft_pf<T, N, true>, y_pf_bytes<T, N, true>(), y_pf_groups<T, N, true>(s), NT, &s->grid_y[0]) ||
+                   persistent_grid(k_yfft_pf<T, N, false>, y_pf_bytes<T, N, false>(), y_pf_groups<T, N, false>(s), NT,
+                                   &s->grid_y[1])
+               ? -1
+               : 0;
+}
+
+template <typename T, int N, bool FWD>
+int launch_x_ct(const Ppe *s, const T *in, size_t in_off, size_t in_sj, size_t in_sk, T *out, size_t out_off,
+                size_t out_sj, size_t out_sk, T scale, cudaStream_t st, const PressureUpdate *pu, bool *fused)
+{
+    using V = typename cplx_of<T>::type;
     const V *tw = reinterpret_cast<const V *>(sizeof(T) == 8 ? (const void *)s->d_twx64 : (const void *)s->d_twx32);
     const size_t sk = (size_t)N * s->ny;
     const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
+    *fused = false;
     if (aligned && in_off == 0 && out_off == 0 && in_sj == (size_t)N && out_sj == (size_t)N && in_sk == sk &&
         out_sk == sk) {
-        constexpr int NT = pf_x_threads<T>(), NBP = pf_x_lines<T, N>();
-        const int total = ((s->ny / 2 + NBP - 1) / NBP) * s->nz;
+        constexpr int NT = pf_x_threads<T>();
+        const int groups = x_pf_groups<T, N>(s);
         if constexpr (sizeof(T) == 4 && !FWD) {
             if (pu != nullptr) {
-                const size_t shmp = sizeof(V) * (size_t)pf_x_smem_elems<T, N>() + pf_x_pu_bytes<T, N>();
-                auto kern = k_xfft_pf<T, N, false, true>;
-                if (shmp > 48 * 1024)
-                    PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmp));
-                kern<<<persistent_grid(kern, shmp, total, NT), NT, shmp, st>>>(in, out, tw, s->ny, total, scale, *pu);
-                PL_CHECK_LAUNCH();
                 *fused = true;
+                PL_CUDA_TRY(launch_chained(k_xfft_pf<T, N, false, true>, s->grid_x[2], NT,
+                                           x_pf_bytes<T, N>() + pf_x_pu_bytes<T, N>(), st, in, out, tw, s->ny, groups,
+                                           scale, *pu));
                 return 0;
             }
         }
-        const size_t shmp = sizeof(V) * (size_t)pf_x_smem_elems<T, N>();
-        if (shmp > 48 * 1024)
-            PL_CUDA_TRY(
-                cudaFuncSetAttribute(k_xfft_pf<T, N, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmp));
-        k_xfft_pf<T, N, FWD><<<persistent_grid(k_xfft_pf<T, N, FWD>, shmp, total, NT), NT, shmp, st>>>(
-            in, out, tw, s->ny, total, scale, PressureUpdate{});
-        PL_CHECK_LAUNCH();
-        *fused = false;
+        PL_CUDA_TRY(launch_chained(k_xfft_pf<T, N, FWD>, s->grid_x[FWD ? 0 : 1], NT, x_pf_bytes<T, N>(), st, in, out,
+                                   tw, s->ny, groups, scale, PressureUpdate{}));
         return 0;
     }
-    if (shm > 48 * 1024)
-        PL_CUDA_TRY(cudaFuncSetAttribute(k_xfft_ct<T, N, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-    dim3 grid((s->ny / 2 + NB - 1) / NB, s->nz);
-    k_xfft_ct<T, N, FWD><<<grid, 256, shm, st>>>(in, in_off, in_sj, in_sk, out, out_off, out_sj, out_sk, tw, s->ny,
-                                                 scale);
-    PL_CHECK_LAUNCH();
+    constexpr int NB = ct_x_lines<N>();
+    PL_CUDA_TRY(launch_chained(k_xfft_ct<T, N, FWD>, dim3((s->ny / 2 + NB - 1) / NB, s->nz), 256, x_ct_bytes<T, N>(), st,
+                               in, in_off, in_sj, in_sk, out, out_off, out_sj, out_sk, tw, s->ny, scale));
     return 0;
 }
 
 template <typename T, int N, bool FWD> int launch_y_ct(const Ppe *s, T *data, cudaStream_t st)
 {
     using V = typename cplx_of<T>::type;
-    constexpr int W = pf_y_cols<V, N, FWD>();
-    const size_t shm = sizeof(V) * (size_t)pf_y_smem_elems<T, N, FWD>();
-    if (shm > 48 * 1024)
-        PL_CUDA_TRY(cudaFuncSetAttribute(k_yfft_pf<T, N, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
     const V *tw = reinterpret_cast<const V *>(sizeof(T) == 8 ? (const void *)s->d_twy64 : (const void *)s->d_twy32);
-    const int total = ((s->nx / 2 + W - 1) / W) * s->nz;
-    k_yfft_pf<T, N, FWD><<<persistent_grid(k_yfft_pf<T, N, FWD>, shm, total, pf_y_threads<T>()), pf_y_threads<T>(), shm,
-                           st>>>(data, tw, s->nx, total);
-    PL_CHECK_LAUNCH();
+    PL_CUDA_TRY(launch_chained(k_yfft_pf<T, N, FWD>, s->grid_y[FWD ? 0 : 1], pf_y_threads<T>(), y_pf_bytes<T, N, FWD>(),
+                               st, data, tw, s->nx, y_pf_groups<T, N, FWD>(s)));
     return 0;
 }
 
 template <typename T, int N> int launch_xdiv(Ppe *s, const DivIn &d, T *out, double *part, cudaStream_t st)
 {
     using V = typename cplx_of<T>::type;
-    constexpr int shm = xdiv_smem_bytes<T, N>();
     const V *tw = reinterpret_cast<const V *>(sizeof(T) == 8 ? (const void *)s->d_twx64 : (const void *)s->d_twx32);
-    if (shm > 48 * 1024)
-        PL_CUDA_TRY(cudaFuncSetAttribute(k_xfft_div_pf<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
-    const int total = ((s->ny / 2 + xdiv_lines(N) - 1) / xdiv_lines(N)) * s->nz;
-    k_xfft_div_pf<T, N><<<persistent_grid(k_xfft_div_pf<T, N>, shm, total, XDIV_THREADS), XDIV_THREADS, shm, st>>>(
-        d, out, tw, s->ny, total, part);
-    PL_CHECK_LAUNCH();
+    PL_CUDA_TRY(launch_chained(k_xfft_div_pf<T, N>, s->grid_x[3], XDIV_THREADS, xdiv_smem_bytes<T, N>(), st, d, out, tw,
+                               s->ny, xdiv_groups<N>(s), part));
     return 0;
 }
 
 #define PL_FFT_INSTANTIATE_T(T, n)                                                                                     \
+    template int prepare_x_ct<T, n>(Ppe *);                                                                            \
+    template int prepare_y_ct<T, n>(Ppe *);                                                                            \
     template int launch_x_ct<T, n, true>(const Ppe *, const T *, size_t, size_t, size_t, T *, size_t, size_t, size_t,  \
                                          T, cudaStream_t, const PressureUpdate *, bool *);                             \
     template int launch_x_ct<T, n, false>(const Ppe *, const T *, size_t, size_t, size_t, T *, size_t, size_t, size_t, \

@@ -28,14 +28,9 @@ inline int sm_count()
     return n;
 }
 
-template <typename K> int persistent_grid(K kernel, size_t shm, int total, int threads = 256)
-{
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, shm) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    return std::max(1, std::min(total, per_sm * sm_count()));
-}
-
+// per plan: shared-memory limits and persistent grids of the kernels below
+template <typename T, int N> int prepare_x_ct(Ppe *s);
+template <typename T, int N> int prepare_y_ct(Ppe *s);
 // x transform (fused: whether the pressure update ran with it)
 template <typename T, int N, bool FWD>
 int launch_x_ct(const Ppe *s, const T *in, size_t in_off, size_t in_sj, size_t in_sk, T *out, size_t out_off,

@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(256) k_xfft(const T *__restrict__ in, size_t i
                                               T *__restrict__ out, size_t out_off, size_t out_sj, size_t out_sk,
                                               FftPlanDev<typename cplx_of<T>::type> plan, int ny, int pb, T scale)
 {
+    pdl_enter();
     using V = typename cplx_of<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = plan.n; // = nx
@@ -91,6 +92,7 @@ template <typename T, bool FWD>
 __global__ void __launch_bounds__(256) k_yfft(T *__restrict__ data, FftPlanDev<typename cplx_of<T>::type> plan,
                                               int nx, int w)
 {
+    pdl_enter();
     using V = typename cplx_of<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = plan.n; // = ny
@@ -144,6 +146,7 @@ __device__ __forceinline__ void pressure_update(const PressureUpdate &pu, size_t
 
 __global__ void __launch_bounds__(256) k_pressure_update(const float *__restrict__ dp, PressureUpdate pu, size_t n)
 {
+    pdl_enter();
     for (size_t o = (size_t)blockIdx.x * 256 + threadIdx.x; o < n; o += (size_t)gridDim.x * 256)
         pressure_update(pu, o, __ldg(dp + o));
 }
@@ -226,6 +229,7 @@ __device__ __forceinline__ void thomas_column(const T *xin, double *xs, TO *xout
 template <typename T>
 __global__ void __launch_bounds__(128) k_thomas(const T *xin, double *xs, T *xout, TridDev t, const double *mode0)
 {
+    pdl_enter();
     const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y;
     if (px >= t.nx) return;
     const size_t col = (size_t)px + (size_t)t.nx * py, stride = (size_t)t.nx * t.ny;
@@ -315,6 +319,7 @@ template <typename T, bool TALL, typename TO = T, bool GAUGE = true, bool RAGGED
 __global__ void __launch_bounds__(TTM_THREADS, 1)
     k_thomas_tmem(const T *xin, TO *xout, double *xsc, TridDev t, const double *mode0, int rounds, uint32_t tcols)
 {
+    pdl_enter();
     constexpr int G = TTM_G, NS = TTM_NS, NT = TTM_THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *cring = reinterpret_cast<double *>(smem_raw);          // [NS][G][NT] mult (fwd) / rb (bwd)
@@ -534,6 +539,7 @@ __global__ void __launch_bounds__(2 * TTM_THREADS, 1)
                 int nx, int ny, int nz, int ncx, int ncy, long long tcs, const double *mode0, int rounds,
                 uint32_t tcols)
 {
+    pdl_enter();
     constexpr int G = TTW_G, NS = TTH_NS, NC = TTM_THREADS, NT = 2 * NC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *cring = reinterpret_cast<double *>(smem_raw);          // [NS][G][NT] tables
@@ -769,6 +775,7 @@ __global__ void __launch_bounds__(2 * TTM_THREADS, 2)
                 int nx, int ny, int nz, int ncx, int ncy, long long tcs, const double *mode0, int rounds,
                 uint32_t tcols)
 {
+    pdl_enter();
     constexpr int G = TTW_G, NS = TTH_NS, NC = TTM_THREADS, NT = 2 * NC, CW = TTH2_CW, CH = TTH2_CH;
     constexpr int SLOT = (int)tth2_slot_bytes();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1048,6 +1055,7 @@ template <typename T>
 __global__ void __launch_bounds__(1024) k_pdd_par(const T *xin, double *xs, T *xout, TridDev t, PddDev p,
                                                   const double *mode0)
 {
+    pdl_enter();
     const int m = threadIdx.y;
     const int q = blockIdx.x * 32 + threadIdx.x, ncol = t.nx * t.ny;
     const bool valid = q < ncol;
@@ -1107,6 +1115,7 @@ template <typename T, int B>
 __global__ void __launch_bounds__(256) k_pdd_tm(const T *xin, T *xout, TridDev t, PddDev p, const double *mode0,
                                                 int kmax, uint32_t tcols)
 {
+    pdl_enter();
     constexpr int G = PTM_G, H = B / G;
     __shared__ double edge[2][8][32]; // [first / last local value][partition][column]
     __shared__ uint32_t tslot;
@@ -1367,6 +1376,34 @@ template <typename V> static void set_plan(FftPlanDev<V> &p, int n, const int *r
     p.tw = tw;
 }
 
+// the plan's grids of the transform kernels compiled for its lengths
+template <typename T> static int prepare_ct(Ppe *s)
+{
+    int rc = 0;
+    switch (s->nx) {
+#define PL_PREP_CASE(n)                                                                                               \
+    case n:                                                                                                          \
+        rc = prepare_x_ct<T, n>(s);                                                                                  \
+        break;
+        PL_FFT_CT_SIZES(PL_PREP_CASE)
+#undef PL_PREP_CASE
+    default:
+        break;
+    }
+    if (rc) return rc;
+    switch (s->ny) {
+#define PL_PREP_CASE(n)                                                                                               \
+    case n:                                                                                                          \
+        rc = prepare_y_ct<T, n>(s);                                                                                  \
+        break;
+        PL_FFT_CT_SIZES(PL_PREP_CASE)
+#undef PL_PREP_CASE
+    default:
+        break;
+    }
+    return rc;
+}
+
 int ppe_create(Ppe *s, int nx, int ny, int nz, double dx, double dy, const double *dzf_global, int nparts,
                int prec)
 {
@@ -1456,6 +1493,7 @@ int ppe_create(Ppe *s, int nx, int ny, int nz, double dx, double dy, const doubl
         s->scratch_elems = (size_t)nx * ny * nz;
         PL_CUDA_TRY(cudaMalloc(&s->d_scratch, sizeof(double) * s->scratch_elems));
     }
+    if (prec == PREC_FP64 ? prepare_ct<double>(s) : prepare_ct<float>(s)) return -1;
     // kernels with > 48 KB of dynamic shared memory
     PL_CUDA_TRY(cudaFuncSetAttribute(k_yfft<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     PL_CUDA_TRY(cudaFuncSetAttribute(k_yfft<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -1579,7 +1617,7 @@ template <typename T> static int launch_pressure_update(const Ppe *s, const T *d
     }
     const size_t n = (size_t)s->nx * s->ny * s->nz;
     const int grid = (int)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 16);
-    k_pressure_update<<<grid, 256, 0, st>>>(reinterpret_cast<const float *>(dp), *pu, n);
+    PL_CUDA_TRY(launch_chained(k_pressure_update, grid, 256, 0, st, reinterpret_cast<const float *>(dp), *pu, n));
     PL_CHECK_LAUNCH();
     return 0;
 }
@@ -1613,11 +1651,9 @@ static int launch_x(const Ppe *s, bool fwd, const T *in, size_t in_off, size_t i
     const FftPlanDev<V> &plan = *reinterpret_cast<const FftPlanDev<V> *>(
         sizeof(T) == 8 ? (const void *)&s->px64 : (const void *)&s->px32);
     if (fwd)
-        k_xfft<T, true><<<grid, 256, shm, st>>>(in, in_off, in_sj, in_sk, out, out_off, out_sj, out_sk, plan, s->ny,
-                                                pb, scale);
+        PL_CUDA_TRY(launch_chained(k_xfft<T, true>, grid, 256, shm, st, in, in_off, in_sj, in_sk, out, out_off, out_sj, out_sk, plan, s->ny, pb, scale));
     else
-        k_xfft<T, false><<<grid, 256, shm, st>>>(in, in_off, in_sj, in_sk, out, out_off, out_sj, out_sk, plan,
-                                                 s->ny, pb, scale);
+        PL_CUDA_TRY(launch_chained(k_xfft<T, false>, grid, 256, shm, st, in, in_off, in_sj, in_sk, out, out_off, out_sj, out_sk, plan, s->ny, pb, scale));
     PL_CHECK_LAUNCH();
     return pu ? launch_pressure_update(s, out, pu, st) : 0;
 }
@@ -1642,9 +1678,9 @@ template <typename T> static int launch_y(const Ppe *s, bool fwd, T *data, cudaS
     const FftPlanDev<V> &plan = *reinterpret_cast<const FftPlanDev<V> *>(
         sizeof(T) == 8 ? (const void *)&s->py64 : (const void *)&s->py32);
     if (fwd)
-        k_yfft<T, true><<<grid, 256, shm, st>>>(data, plan, s->nx, w);
+        PL_CUDA_TRY(launch_chained(k_yfft<T, true>, grid, 256, shm, st, data, plan, s->nx, w));
     else
-        k_yfft<T, false><<<grid, 256, shm, st>>>(data, plan, s->nx, w);
+        PL_CUDA_TRY(launch_chained(k_yfft<T, false>, grid, 256, shm, st, data, plan, s->nx, w));
     PL_CHECK_LAUNCH();
     return 0;
 }
@@ -1670,9 +1706,7 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
                 uint32_t tcols = 32;
                 while (tcols < (uint32_t)s->nz) tcols *= 2;
                 PL_CUDA_TRY(cudaFuncSetAttribute(k_thomas_th2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-                k_thomas_th2<<<ctas2, 2 * TTM_THREADS, shm, st>>>(x, x, s->d_tmult, s->d_trb, s->d_a, s->d_c, s->nx,
-                                                                   s->ny, s->nz, s->ncx, s->ncy, (long long)s->tcs,
-                                                                   mode0, rounds2, tcols);
+                PL_CUDA_TRY(launch_chained(k_thomas_th2, ctas2, 2 * TTM_THREADS, shm, st, x, x, s->d_tmult, s->d_trb, s->d_a, s->d_c, s->nx, s->ny, s->nz, s->ncx, s->ncy, (long long)s->tcs, mode0, rounds2, tcols));
                 PL_CHECK_LAUNCH();
                 return 0;
             }
@@ -1681,9 +1715,7 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
         uint32_t tcols = 32;
         while (tcols < 2u * (uint32_t)s->nz) tcols *= 2;
         PL_CUDA_TRY(cudaFuncSetAttribute(k_thomas_th<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        k_thomas_th<T><<<ctas1, 2 * TTM_THREADS, shm, st>>>(x, x, s->d_tmult, s->d_trb, s->d_a, s->d_c, s->nx, s->ny,
-                                                              s->nz, s->ncx, s->ncy, (long long)s->tcs, mode0, rounds1,
-                                                              tcols);
+        PL_CUDA_TRY(launch_chained(k_thomas_th<T>, ctas1, 2 * TTM_THREADS, shm, st, x, x, s->d_tmult, s->d_trb, s->d_a, s->d_c, s->nx, s->ny, s->nz, s->ncx, s->ncy, (long long)s->tcs, mode0, rounds1, tcols));
         PL_CHECK_LAUNCH();
         return 0;
     }
@@ -1704,9 +1736,9 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
         auto kern = tall ? (ragged ? k_thomas_tmem<T, true, T, true, true> : k_thomas_tmem<T, true>)
                          : (ragged ? k_thomas_tmem<T, false, T, true, true> : k_thomas_tmem<T, false>);
         PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        kern<<<ctas, TTM_THREADS, shm, st>>>(x, x, xsc, t, mode0, rounds, tcols);
+        PL_CUDA_TRY(launch_chained(kern, ctas, TTM_THREADS, shm, st, x, x, xsc, t, mode0, rounds, tcols));
     } else if (s->nparts == 0) {
-        k_thomas<T><<<grid, 128, 0, st>>>(x, xs, x, t, mode0);
+        PL_CUDA_TRY(launch_chained(k_thomas<T>, grid, 128, 0, st, x, xs, x, t, mode0));
     } else if (s->nparts <= 32) {
         PddDev p{};
         p.nparts = s->nparts;
@@ -1735,11 +1767,9 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
             auto kern = groups2 ? k_pdd_tm<T, 2 * PTM_G> : k_pdd_tm<T, PTM_G>;
             if (dyn > 48 * 1024)
                 PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-            kern<<<(ncol + 31) / 32, dim3(32, s->nparts), dyn, st>>>(x, x, t, p, sizeof(T) == 4 ? mode0 : nullptr, kmax,
-                                                                      tcols);
+            PL_CUDA_TRY(launch_chained(kern, (ncol + 31) / 32, dim3(32, s->nparts), dyn, st, x, x, t, p, sizeof(T) == 4 ? mode0 : nullptr, kmax, tcols));
         } else {
-            k_pdd_par<T><<<(ncol + 31) / 32, dim3(32, s->nparts), 0, st>>>(x, s->d_scratch, x, t, p,
-                                                                          sizeof(T) == 4 ? mode0 : nullptr);
+            PL_CUDA_TRY(launch_chained(k_pdd_par<T>, (ncol + 31) / 32, dim3(32, s->nparts), 0, st, x, s->d_scratch, x, t, p, sizeof(T) == 4 ? mode0 : nullptr));
         }
     } else {
         if (sizeof(T) == 4) {

@@ -61,6 +61,11 @@ struct Ppe {
     int slab = 0, has_up = 0, has_down = 0;
     double *d_tvar = nullptr, *d_y1 = nullptr, *d_y2 = nullptr, *d_y3 = nullptr;
 
+    // grids of the persistent transform kernels (occupancy of the plan's
+    // kernels, found once): x forward, inverse, inverse with the pressure
+    // update, calcRHS + forward; y forward, inverse
+    int grid_x[4] = {0, 0, 0, 0}, grid_y[2] = {0, 0};
+
     // optional per-launch marker (profiling): called after every kernel launch
     void (*mark)(void *ctx, const char *name) = nullptr;
     void *mark_ctx = nullptr;

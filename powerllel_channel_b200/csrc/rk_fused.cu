@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(FT, 2) k_rk_fused(const double *__restrict__ u
                                                    double *__restrict__ vo, double *__restrict__ wo, StepParams p,
                                                    MeshDev m, FConst K, MeanRed red, int kchunk)
 {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *ur = reinterpret_cast<double *>(smem_raw); // u, v, w
     double *sr = ur + 3 * FSS;                         // u1, v1, w1
@@ -443,24 +444,35 @@ int rk_fused_blocks(const StepParams &p)
     return (int)(t.x * t.y) * ((p.nz + 1) / 2);
 }
 
-int launch_rk_fused_fp64(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
-                         const StepParams &p, const MeshDev &m, MeanState &ms, cudaStream_t st)
+static size_t fused_smem() { return sizeof(double) * (6 * FSS + 8 * (F_KCHUNK + 4)); }
+
+int rk_prepare(const void *kern, int threads, size_t shm, dim3 tiles, int nz, int most, RkLaunch *out)
 {
-    const size_t shm = sizeof(double) * (6 * FSS + 8 * (F_KCHUNK + 4));
-    // u_crf == 0 (the channel's usual frame) drops the frame-velocity terms
-    auto kern = (p.u_crf != 0.0) ? k_rk_fused<true> : k_rk_fused<false>;
     PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
     // prefer the largest shared-memory carve-out: two CTAs per SM
     PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                      (int)cudaSharedmemCarveoutMaxShared));
     int per_sm = 0, dev = 0, nsm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FT, shm) != cudaSuccess || per_sm < 1) per_sm = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, shm) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    dim3 grid = fused_tiles(p);
-    const int kchunk = rk_kchunk((long)grid.x * grid.y, p.nz, F_KCHUNK, per_sm * (nsm > 0 ? nsm : 1));
-    grid.z = (p.nz + kchunk - 1) / kchunk;
-    if ((int)(grid.x * grid.y * grid.z) > ms.max_blocks) {
+    out->kchunk = rk_kchunk((long)tiles.x * tiles.y, nz, most, per_sm * (nsm > 0 ? nsm : 1));
+    out->grid = dim3(tiles.x, tiles.y, (nz + out->kchunk - 1) / out->kchunk);
+    return 0;
+}
+
+// u_crf == 0 (the channel's usual frame) drops the frame-velocity terms
+int rk_fused_prepare(const StepParams &p, RkLaunch *out)
+{
+    return rk_prepare(p.u_crf != 0.0 ? (const void *)k_rk_fused<true> : (const void *)k_rk_fused<false>, FT, fused_smem(),
+                      fused_tiles(p), p.nz, F_KCHUNK, out);
+}
+
+int launch_rk_fused_fp64(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
+                         const StepParams &p, const MeshDev &m, MeanState &ms, const RkLaunch &l, cudaStream_t st)
+{
+    if ((int)(l.grid.x * l.grid.y * l.grid.z) > ms.max_blocks) {
         set_error("mean buffer too small for the fused RK kernel");
         return -1;
     }
@@ -475,8 +487,8 @@ int launch_rk_fused_fp64(const double *u, const double *v, const double *w, doub
     K.ucx = 0.5 * p.dt * p.u_crf * p.dx_inv;
     for (int q = 0; q < 3; q++) K.fb[q] = p.dt * p.fb[q];
     MeanRed r{ms.partial, ms.counter, ms.scalar, (double)p.nx, (double)p.ny, ms.vel_force};
-    kern<<<grid, dim3(FX, FT / FX), shm, st>>>(u, v, w, uo, vo, wo, p, m, K, r, kchunk);
-    PL_CHECK_LAUNCH();
+    PL_CUDA_TRY(launch_chained(p.u_crf != 0.0 ? k_rk_fused<true> : k_rk_fused<false>, l.grid, dim3(FX, FT / FX),
+                               fused_smem(), st, u, v, w, uo, vo, wo, p, m, K, r, l.kchunk));
     return 0;
 }
 

@@ -232,6 +232,7 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
                                                    MeshDev m, MConst K, MeanRed red, int kchunk,
                                                    const float *__restrict__ pq, int pinc)
 {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2 *stg = reinterpret_cast<double2 *>(smem_raw);    // FP64 staging, [field][pair]
     float *ur = reinterpret_cast<float *>(stg + 3 * MPAIRS); // u, v, w rings, two planes
@@ -487,23 +488,22 @@ int rk_mixed_blocks(const StepParams &p)
     return (int)(t.x * t.y) * ((p.nz + 1) / 2);
 }
 
-int launch_rk_mixed(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
-                    const StepParams &p, const MeshDev &m, MeanState &ms, const float *pq, int pinc, cudaStream_t st)
+static size_t mixed_smem()
 {
-    const size_t shm = sizeof(double2) * 3 * MPAIRS + sizeof(float) * 4 * MSS + (sizeof(float4) * 2 + sizeof(double)) * (MX_KCHUNK + 4);
-    auto kern = (p.u_crf != 0.0) ? k_rk_mixed<true> : k_rk_mixed<false>;
-    PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-    PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared));
-    int per_sm = 0, dev = 0, nsm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MT, shm) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    dim3 grid = mixed_tiles(p);
-    const int kchunk = rk_kchunk((long)grid.x * grid.y, p.nz, MX_KCHUNK, per_sm * (nsm > 0 ? nsm : 1));
-    grid.z = (p.nz + kchunk - 1) / kchunk;
-    if ((int)(grid.x * grid.y * grid.z) > ms.max_blocks) {
+    return sizeof(double2) * 3 * MPAIRS + sizeof(float) * 4 * MSS + (sizeof(float4) * 2 + sizeof(double)) * (MX_KCHUNK + 4);
+}
+
+int rk_mixed_prepare(const StepParams &p, RkLaunch *out)
+{
+    return rk_prepare(p.u_crf != 0.0 ? (const void *)k_rk_mixed<true> : (const void *)k_rk_mixed<false>, MT, mixed_smem(),
+                      mixed_tiles(p), p.nz, MX_KCHUNK, out);
+}
+
+int launch_rk_mixed(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
+                    const StepParams &p, const MeshDev &m, MeanState &ms, const float *pq, int pinc, const RkLaunch &l,
+                    cudaStream_t st)
+{
+    if ((int)(l.grid.x * l.grid.y * l.grid.z) > ms.max_blocks) {
         set_error("mean buffer too small for the mixed fused RK kernel");
         return -1;
     }
@@ -518,8 +518,8 @@ int launch_rk_mixed(const double *u, const double *v, const double *w, double *u
     K.ncc = both(-2.0 * p.dt * p.re_inv * (p.dx_inv * p.dx_inv + p.dy_inv * p.dy_inv));
     K.nucx = both(-0.5 * p.dt * p.u_crf * p.dx_inv);
     MeanRed r{ms.partial, ms.counter, ms.scalar, (double)p.nx, (double)p.ny, ms.vel_force};
-    kern<<<grid, dim3(MX, MT / MX), shm, st>>>(u, v, w, uo, vo, wo, p, m, K, r, kchunk, pq, pinc);
-    PL_CHECK_LAUNCH();
+    PL_CUDA_TRY(launch_chained(p.u_crf != 0.0 ? k_rk_mixed<true> : k_rk_mixed<false>, l.grid, dim3(MX, MT / MX),
+                               mixed_smem(), st, u, v, w, uo, vo, wo, p, m, K, r, l.kchunk, pq, pinc));
     return 0;
 }
 

@@ -548,6 +548,7 @@ __global__ void __launch_bounds__(RHS_BX *RHS_BY) k_correct_force(const TP *__re
                                                                    double *w, StepParams p, MeshDev m, int forced_x,
                                                                    const double *scalar)
 {
+    pdl_enter();
     using P2 = typename PairOf<TP>::type;
     const int i = 2 * (blockIdx.x * RHS_BX + threadIdx.x);
     const int j = blockIdx.y * RHS_BY + threadIdx.y;
@@ -595,6 +596,7 @@ __global__ void __launch_bounds__(RHS_BX *RHS_BY) k_correct_force(const TP *__re
 // per-plane sums of the warp partials (fixed order): mode0[k] = sum_ij r
 __global__ void k_plane_sums(const double *part, int nper, int nz, double *mode0)
 {
+    pdl_enter();
     const int k = blockIdx.x;
     if (k >= nz) return;
     double s = 0.0;
@@ -779,16 +781,16 @@ int launch_rk2m_fp64(double *u, double *v, double *w, const double *u1, const do
 int launch_correct_force_fp64(const double *p_, double *u, double *v, double *w, const StepParams &p,
                               const MeshDev &m, int forced_x, const double *scalar, cudaStream_t st)
 {
-    k_correct_force<double><<<rhs_mixed_grid(p), dim3(RHS_BX, RHS_BY), 0, st>>>(p_, u, v, w, p, m, forced_x, scalar);
-    PL_CHECK_LAUNCH();
+    PL_CUDA_TRY(launch_chained(k_correct_force<double>, rhs_mixed_grid(p), dim3(RHS_BX, RHS_BY), 0, st, p_, u, v, w, p, m,
+                               forced_x, scalar));
     return 0;
 }
 
 int launch_correct_force_f32(const float *p_, double *u, double *v, double *w, const StepParams &p, const MeshDev &m,
                              int forced_x, const double *scalar, cudaStream_t st)
 {
-    k_correct_force<float><<<rhs_mixed_grid(p), dim3(RHS_BX, RHS_BY), 0, st>>>(p_, u, v, w, p, m, forced_x, scalar);
-    PL_CHECK_LAUNCH();
+    PL_CUDA_TRY(launch_chained(k_correct_force<float>, rhs_mixed_grid(p), dim3(RHS_BX, RHS_BY), 0, st, p_, u, v, w, p, m,
+                               forced_x, scalar));
     return 0;
 }
 
@@ -822,8 +824,7 @@ int warp_partials_per_plane(const StepParams &p)
 
 int launch_plane_sums(const double *part, int nper, int nz, double *mode0, cudaStream_t st)
 {
-    k_plane_sums<<<nz, 256, 0, st>>>(part, nper, nz, mode0);
-    PL_CHECK_LAUNCH();
+    PL_CUDA_TRY(launch_chained(k_plane_sums, nz, 256, 0, st, part, nper, nz, mode0));
     return 0;
 }
 

@@ -55,19 +55,28 @@ struct MeanState {
 };
 
 // fused RK1 + RK2 (rk_fused.cu): u -> (uo, vo, wo) out of place
+struct RkLaunch { // found once per channel
+    dim3 grid;
+    int kchunk = 0; // planes per CTA
+};
 int rk_fused_blocks(const StepParams &p);
+int rk_fused_prepare(const StepParams &p, RkLaunch *out);
 int launch_rk_fused_fp64(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
-                         const StepParams &p, const MeshDev &m, MeanState &ms, cudaStream_t st);
+                         const StepParams &p, const MeshDev &m, MeanState &ms, const RkLaunch &l, cudaStream_t st);
 
 // mixed path: both RK stages in FP32 flux form (rk_mixed.cu); with pinc,
 // u_hat = u* - dt G pq is stored (pq: the FP32 pressure prediction,
 // interior-only layout), whose divergence / dt is the increment's residual
 int rk_mixed_blocks(const StepParams &p);
+int rk_mixed_prepare(const StepParams &p, RkLaunch *out);
 int launch_rk_mixed(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
-                    const StepParams &p, const MeshDev &m, MeanState &ms, const float *pq, int pinc, cudaStream_t st);
+                    const StepParams &p, const MeshDev &m, MeanState &ms, const float *pq, int pinc, const RkLaunch &l,
+                    cudaStream_t st);
 // planes per z-chunk of the fused RK kernels (at most `most`) for a grid of
 // `tiles` tile columns, `resident` CTAs fitting the chip at once
 int rk_kchunk(long tiles, int nz, int most, int resident);
+// the kernel's shared-memory settings and launch shape
+int rk_prepare(const void *kern, int threads, size_t shm, dim3 tiles, int nz, int most, RkLaunch *out);
 
 int launch_rk2m_fp64(double *u, double *v, double *w, const double *u1, const double *v1, const double *w1,
                      const StepParams &p, const MeshDev &m, MeanState &ms, cudaStream_t st);
