@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "channel.cuh"
+#include "fft.cuh" // cp.async helpers
 #include "stencil_rhs.cuh"
 
 using namespace pl;
@@ -50,91 +51,191 @@ dim3 adj_grid(const StepParams &p) { return dim3((p.nx + 63) / 64, (p.ny + 3) / 
 // of w; Pyz: z flux of v and y flux of w) gets one adjoint, the sum of the
 // adjoints of its two uses; the adjoint of a flux difference
 // -0.25 (F(o) - F(o-1)) h_o is -0.25 (h_o r(o) - h_{o+1} r(o+1)).
-__global__ void __launch_bounds__(256) k_adj_rk(const double *__restrict__ u, const double *__restrict__ v,
+//
+// 2.5D blocking as in the fused RK kernel: a CTA marches a 32 x 8 tile up a
+// chunk of planes, with three-plane shared-memory rings of the six fields
+// (halo 1 of 2 stored, so that copies are aligned pairs), one barrier per
+// plane.  What a point needs of the plane below are the terms of the face
+// between, which are those of that plane's upper face and stay in registers,
+// as do the values above, the next plane's centre values: 30 shared loads a
+// point.  A kernel of a point per thread, reading its 47 operands from L1 and
+// L2, took 280 us at 256x192x128; this one takes 149, and 186 with the second
+// operand e (4.1 and 3.9 TB/s at 96 and 120 B/point).
+constexpr int AX = 32, AY = 8, AW = AX + 4, AH = AY + 4, APS = AW * AH, AT = AX * AY, ASS = 6 * APS;
+
+__global__ void __launch_bounds__(AT, 2) k_adj_rk(const double *__restrict__ u, const double *__restrict__ v,
                                                 const double *__restrict__ w, const double *__restrict__ ru,
                                                 const double *__restrict__ rv, const double *__restrict__ rw,
                                                 const double *__restrict__ eu, const double *__restrict__ ev,
                                                 const double *__restrict__ ew, double *__restrict__ ou,
                                                 double *__restrict__ ov, double *__restrict__ ow, double alpha,
-                                                double beta, double gamma, StepParams p, MeshDev m)
+                                                double beta, double gamma, StepParams p, MeshDev m, int kchunk)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z + 1;
-    if (i >= p.nx || j >= p.ny) return;
-    const Nb n = neighbours(i, j, k, p.nx, p.ny);
+    extern __shared__ __align__(16) double ring[]; // [slot][u v w ru rv rw][xy]
+    const int lane = threadIdx.x, wid = threadIdx.y, tid = lane + AX * wid;
+    const int i0 = blockIdx.x * AX, j0 = blockIdx.y * AY;
+    const int kbeg = blockIdx.z * kchunk + 1, kend = min(kbeg + kchunk - 1, p.nz);
+    const size_t sk = (size_t)p.nx * p.ny;
+
+    // copies: 12 rows of 18 aligned pairs per field and plane, a pair of each
+    // field per thread; x and y wrap, nx is even
+    constexpr int PAIRS = AH * (AW / 2);
+    static_assert(PAIRS <= AT, "one pair per thread");
+    const int cr = tid / (AW / 2), cc = tid % (AW / 2);
+    const size_t soff = tid < PAIRS ? (size_t)((j0 - 2 + cr + p.ny) % p.ny) * p.nx + (i0 - 2 + 2 * cc + p.nx) % p.nx : 0;
+    auto issue = [&](int k, int slot) {
+        if (tid < PAIRS) {
+            double *d = ring + slot * ASS + cr * AW + 2 * cc;
+            const size_t o = sk * k + soff;
+            cp_async_16(d, u + o);
+            cp_async_16(d + APS, v + o);
+            cp_async_16(d + 2 * APS, w + o);
+            cp_async_16(d + 3 * APS, ru + o);
+            cp_async_16(d + 4 * APS, rv + o);
+            cp_async_16(d + 5 * APS, rw + o);
+        }
+        cp_async_commit();
+    };
+    const int i = i0 + lane, j = j0 + wid, xy = (2 + wid) * AW + 2 + lane;
+    const bool inside = i < p.nx && j < p.ny;
+
+    // plane k in slot (k - kbeg + 1) % 3
+    issue(kbeg - 1, 0);
+    issue(kbeg, 1);
+    issue(kbeg + 1, 2);
+    cp_async_wait<0>();
+    __syncthreads();
+
     const double dxi = p.dx_inv, dyi = p.dy_inv, re = p.re_inv, q = 0.25;
-    const double f_c = __ldg(m.dzf + k), f_p = __ldg(m.dzf + k + 1), f_m = __ldg(m.dzf + k - 1);
-    const double ci_c = __ldg(m.dzc_inv + k), ci_m = __ldg(m.dzc_inv + k - 1), ci_p = __ldg(m.dzc_inv + k + 1);
-    const double fi_c = __ldg(m.dzf_inv + k), fi_p = __ldg(m.dzf_inv + k + 1), fi_m = __ldg(m.dzf_inv + k - 1);
-
-    const double Uc = __ldg(u + n.c), Uxp = __ldg(u + n.xp), Uxm = __ldg(u + n.xm), Uyp = __ldg(u + n.yp),
-                 Uzp = __ldg(u + n.zp), Uxmyp = __ldg(u + n.xmyp), Uxmzp = __ldg(u + n.xmzp);
-    const double Vc = __ldg(v + n.c), Vxp = __ldg(v + n.xp), Vym = __ldg(v + n.ym), Vyp = __ldg(v + n.yp),
-                 Vzp = __ldg(v + n.zp), Vxpym = __ldg(v + n.xpym), Vymzp = __ldg(v + n.ymzp);
-    const double Wc = __ldg(w + n.c), Wxp = __ldg(w + n.xp), Wyp = __ldg(w + n.yp), Wzp = __ldg(w + n.zp),
-                 Wzm = __ldg(w + n.zm), Wxpzm = __ldg(w + n.xpzm), Wypzm = __ldg(w + n.ypzm);
-
-    const double RUc = __ldg(ru + n.c), RUxp = __ldg(ru + n.xp), RUxm = __ldg(ru + n.xm), RUyp = __ldg(ru + n.yp),
-                 RUym = __ldg(ru + n.ym), RUzp = __ldg(ru + n.zp), RUzm = __ldg(ru + n.zm),
-                 RUxmyp = __ldg(ru + n.xmyp), RUxmzp = __ldg(ru + n.xmzp);
-    const double RVc = __ldg(rv + n.c), RVxp = __ldg(rv + n.xp), RVxm = __ldg(rv + n.xm), RVyp = __ldg(rv + n.yp),
-                 RVym = __ldg(rv + n.ym), RVzp = __ldg(rv + n.zp), RVzm = __ldg(rv + n.zm),
-                 RVxpym = __ldg(rv + n.xpym), RVymzp = __ldg(rv + n.ymzp);
-    const double RWc = __ldg(rw + n.c), RWxp = __ldg(rw + n.xp), RWxm = __ldg(rw + n.xm), RWyp = __ldg(rw + n.yp),
-                 RWym = __ldg(rw + n.ym), RWzp = __ldg(rw + n.zp), RWzm = __ldg(rw + n.zm),
-                 RWxpzm = __ldg(rw + n.xpzm), RWypzm = __ldg(rw + n.ypzm);
-
-    // flux adjoints at the faces of cell g and of its x-, y- and z-neighbours below
-    const double Aux_c = -q * dxi * (RUc - RUxp), Aux_m = -q * dxi * (RUxm - RUc);
-    const double Avy_c = -q * dyi * (RVc - RVyp), Avy_m = -q * dyi * (RVym - RVc);
-    const double Awz_c = -q * (RWc * ci_c - RWzp * ci_p), Awz_m = -q * (RWzm * ci_m - RWc * ci_c);
-    const double Pxy_c = -q * dyi * (RUc - RUyp) - q * dxi * (RVc - RVxp);
-    const double Pxy_ym = -q * dyi * (RUym - RUc) - q * dxi * (RVym - RVxpym);
-    const double Pxy_xm = -q * dyi * (RUxm - RUxmyp) - q * dxi * (RVxm - RVc);
-    const double Pxz_c = -q * (RUc * fi_c - RUzp * fi_p) - q * dxi * (RWc - RWxp);
-    const double Pxz_zm = -q * (RUzm * fi_m - RUc * fi_c) - q * dxi * (RWzm - RWxpzm);
-    const double Pxz_xm = -q * (RUxm * fi_c - RUxmzp * fi_p) - q * dxi * (RWxm - RWc);
-    const double Pyz_c = -q * (RVc * fi_c - RVzp * fi_p) - q * dyi * (RWc - RWyp);
-    const double Pyz_zm = -q * (RVzm * fi_m - RVc * fi_c) - q * dyi * (RWzm - RWypzm);
-    const double Pyz_ym = -q * (RVym * fi_c - RVymzp * fi_p) - q * dyi * (RWym - RWc);
-
-    // convective part: flux adjoint times the derivative of the flux
-    const double ut_c = (Uc * f_p + Uzp * f_c) * ci_c, ut_xm = (Uxm * f_p + Uxmzp * f_c) * ci_c;
-    const double vt_c = (Vc * f_p + Vzp * f_c) * ci_c, vt_ym = (Vym * f_p + Vymzp * f_c) * ci_c;
-    double su = 2.0 * (Uc + Uxp) * Aux_c + 2.0 * (Uxm + Uc) * Aux_m + (Vc + Vxp) * Pxy_c + (Vym + Vxpym) * Pxy_ym +
-                f_p * ci_c * (Wc + Wxp) * Pxz_c + f_m * ci_m * (Wzm + Wxpzm) * Pxz_zm;
-    double sv = 2.0 * (Vc + Vyp) * Avy_c + 2.0 * (Vym + Vc) * Avy_m + (Uc + Uyp) * Pxy_c + (Uxm + Uxmyp) * Pxy_xm +
-                f_p * ci_c * (Wc + Wyp) * Pyz_c + f_m * ci_m * (Wzm + Wypzm) * Pyz_zm;
-    double sw = 2.0 * (Wc + Wzp) * Awz_c + 2.0 * (Wzm + Wc) * Awz_m + ut_c * Pxz_c + ut_xm * Pxz_xm + vt_c * Pyz_c +
-                vt_ym * Pyz_ym;
-
-    // u_crf advection: adjoint of -0.5 u_crf (q(i+1) - q(i-1)) dx_inv
-    const double hc = 0.5 * p.u_crf * dxi;
-    su -= hc * (RUxm - RUxp);
-    sv -= hc * (RVxm - RVxp);
-    sw -= hc * (RWxm - RWxp);
-
-    // viscous part; the wall ghosts q(0) = 2bc - q(1), q(nz+1) = 2bc - q(nz)
-    // of u and v double the wall-face coefficients
-    const double dxi2 = dxi * dxi, dyi2 = dyi * dyi;
-    const double ca = (k == 1) ? 2.0 : 1.0, cb = (k == p.nz) ? 2.0 : 1.0;
-    su += re * ((RUxp - 2.0 * RUc + RUxm) * dxi2 + (RUyp - 2.0 * RUc + RUym) * dyi2) -
-          cb * ci_c * re * (RUc * fi_c - RUzp * fi_p) + ca * ci_m * re * (RUzm * fi_m - RUc * fi_c);
-    sv += re * ((RVxp - 2.0 * RVc + RVxm) * dxi2 + (RVyp - 2.0 * RVc + RVym) * dyi2) -
-          cb * ci_c * re * (RVc * fi_c - RVzp * fi_p) + ca * ci_m * re * (RVzm * fi_m - RVc * fi_c);
-    sw += re * ((RWxp - 2.0 * RWc + RWxm) * dxi2 + (RWyp - 2.0 * RWc + RWym) * dyi2) -
-          fi_p * re * (RWc * ci_c - RWzp * ci_p) + fi_c * re * (RWzm * ci_m - RWc * ci_c);
-
-    double xu = alpha * RUc + beta * su, xv = alpha * RVc + beta * sv, xw = alpha * RWc + beta * sw;
-    if (eu) {
-        xu += gamma * __ldg(eu + n.c);
-        xv += gamma * __ldg(ev + n.c);
-        xw += gamma * __ldg(ew + n.c);
+    const double dxi2 = dxi * dxi, dyi2 = dyi * dyi, hc = 0.5 * p.u_crf * dxi;
+    // mesh factors of the plane below, this plane and the plane above
+    double f_m, f_c = __ldg(m.dzf + kbeg - 1), f_p = __ldg(m.dzf + kbeg);
+    double ci_m, ci_c = __ldg(m.dzc_inv + kbeg - 1), ci_p = __ldg(m.dzc_inv + kbeg);
+    double fi_c = __ldg(m.dzf_inv + kbeg - 1), fi_p = __ldg(m.dzf_inv + kbeg);
+    // terms of the face below: the z differences of r, the products of the
+    // base state with the flux adjoints
+    double gu_m, gv_m, cw_m, tu_m, tv_m, zw_m;
+    // centre values of plane k, and ru, u at x - 1, rv, v at y - 1
+    double U, V, W, RU, RV, RW, Uxm, Vym, RUxm, RVym;
+    auto above = [&](const double *n) { // n: the point in the plane above
+        U = n[0];
+        V = n[APS];
+        W = n[2 * APS];
+        RU = n[3 * APS];
+        RV = n[4 * APS];
+        RW = n[5 * APS];
+        Uxm = n[-1];
+        Vym = n[APS - AW];
+        RUxm = n[3 * APS - 1];
+        RVym = n[4 * APS - AW];
+    };
+    {
+        const double *c = ring + xy, *n = c + ASS;
+        gu_m = c[3 * APS] * fi_c - n[3 * APS] * fi_p;
+        gv_m = c[4 * APS] * fi_c - n[4 * APS] * fi_p;
+        cw_m = c[5 * APS] * ci_c - n[5 * APS] * ci_p;
+        tu_m = (c[2 * APS] + c[2 * APS + 1]) * (-q * gu_m - q * dxi * (c[5 * APS] - c[5 * APS + 1]));
+        tv_m = (c[2 * APS] + c[2 * APS + AW]) * (-q * gv_m - q * dyi * (c[5 * APS] - c[5 * APS + AW]));
+        zw_m = (c[2 * APS] + n[2 * APS]) * (-q * cw_m);
+        above(n);
     }
-    ou[n.c] = xu;
-    ov[n.c] = xv;
-    ow[n.c] = (k == p.nz) ? 0.0 : xw;
+    int a = 1, b = 2, free = 0; // slots of the planes k, k + 1, k + 2
+    for (int k = kbeg; k <= kend; k++) {
+        __syncthreads(); // everyone is done with the slot of plane k - 1
+        if (k < kend) issue(k + 2, free);
+        f_m = f_c;
+        f_c = f_p;
+        f_p = __ldg(m.dzf + k + 1);
+        ci_m = ci_c;
+        ci_c = ci_p;
+        ci_p = __ldg(m.dzc_inv + k + 1);
+        fi_c = fi_p;
+        fi_p = __ldg(m.dzf_inv + k + 1);
+        const double *c = ring + a * ASS + xy, *n = ring + b * ASS + xy;
+        const double *cv = c + APS, *cw = c + 2 * APS, *cru = c + 3 * APS, *crv = c + 4 * APS, *crw = c + 5 * APS;
+        const double Uc = U, Vc = V, Wc = W, RUc = RU, RVc = RV, RWc = RW;
+        const double Uxm_c = Uxm, Vym_c = Vym, RUxm_c = RUxm, RVym_c = RVym;
+        above(n);
+        const double Uxp = c[1], Uyp = c[AW], Uxmyp = c[AW - 1];
+        const double Vxp = cv[1], Vyp = cv[AW], Vxpym = cv[1 - AW];
+        const double Wxp = cw[1], Wyp = cw[AW];
+        const double RUxp = cru[1], RUyp = cru[AW], RUym = cru[-AW], RUxmyp = cru[AW - 1];
+        const double RVxp = crv[1], RVxm = crv[-1], RVyp = crv[AW], RVxpym = crv[1 - AW];
+        const double RWxp = crw[1], RWxm = crw[-1], RWyp = crw[AW], RWym = crw[-AW];
+
+        // z differences over the face above, here and at x - 1, y - 1
+        const double gu = RUc * fi_c - RU * fi_p, gu_xm = RUxm_c * fi_c - RUxm * fi_p;
+        const double gv = RVc * fi_c - RV * fi_p, gv_ym = RVym_c * fi_c - RVym * fi_p;
+        const double cwz = RWc * ci_c - RW * ci_p;
+        // flux adjoints
+        const double Aux_c = -q * dxi * (RUc - RUxp), Aux_m = -q * dxi * (RUxm_c - RUc);
+        const double Avy_c = -q * dyi * (RVc - RVyp), Avy_m = -q * dyi * (RVym_c - RVc);
+        const double Pxy_c = -q * dyi * (RUc - RUyp) - q * dxi * (RVc - RVxp);
+        const double Pxy_ym = -q * dyi * (RUym - RUc) - q * dxi * (RVym_c - RVxpym);
+        const double Pxy_xm = -q * dyi * (RUxm_c - RUxmyp) - q * dxi * (RVxm - RVc);
+        const double Pxz_c = -q * gu - q * dxi * (RWc - RWxp), Pxz_xm = -q * gu_xm - q * dxi * (RWxm - RWc);
+        const double Pyz_c = -q * gv - q * dyi * (RWc - RWyp), Pyz_ym = -q * gv_ym - q * dyi * (RWym - RWc);
+        const double tu = (Wc + Wxp) * Pxz_c, tv = (Wc + Wyp) * Pyz_c, zw = (Wc + W) * (-q * cwz);
+
+        // convective part: flux adjoint times the derivative of the flux
+        const double ut_c = (Uc * f_p + U * f_c) * ci_c, ut_xm = (Uxm_c * f_p + Uxm * f_c) * ci_c;
+        const double vt_c = (Vc * f_p + V * f_c) * ci_c, vt_ym = (Vym_c * f_p + Vym * f_c) * ci_c;
+        double su = 2.0 * (Uc + Uxp) * Aux_c + 2.0 * (Uxm_c + Uc) * Aux_m + (Vc + Vxp) * Pxy_c +
+                    (Vym_c + Vxpym) * Pxy_ym + f_p * ci_c * tu + f_m * ci_m * tu_m;
+        double sv = 2.0 * (Vc + Vyp) * Avy_c + 2.0 * (Vym_c + Vc) * Avy_m + (Uc + Uyp) * Pxy_c +
+                    (Uxm_c + Uxmyp) * Pxy_xm + f_p * ci_c * tv + f_m * ci_m * tv_m;
+        double sw = 2.0 * (zw + zw_m) + ut_c * Pxz_c + ut_xm * Pxz_xm + vt_c * Pyz_c + vt_ym * Pyz_ym;
+
+        // u_crf advection: adjoint of -0.5 u_crf (q(i+1) - q(i-1)) dx_inv
+        su -= hc * (RUxm_c - RUxp);
+        sv -= hc * (RVxm - RVxp);
+        sw -= hc * (RWxm - RWxp);
+
+        // viscous part; the wall ghosts q(0) = 2bc - q(1), q(nz+1) = 2bc - q(nz)
+        // of u and v double the wall-face coefficients
+        const double ca = (k == 1) ? 2.0 : 1.0, cb = (k == p.nz) ? 2.0 : 1.0;
+        su += re * ((RUxp - 2.0 * RUc + RUxm_c) * dxi2 + (RUyp - 2.0 * RUc + RUym) * dyi2) - cb * ci_c * re * gu +
+              ca * ci_m * re * gu_m;
+        sv += re * ((RVxp - 2.0 * RVc + RVxm) * dxi2 + (RVyp - 2.0 * RVc + RVym_c) * dyi2) - cb * ci_c * re * gv +
+              ca * ci_m * re * gv_m;
+        sw += re * ((RWxp - 2.0 * RWc + RWxm) * dxi2 + (RWyp - 2.0 * RWc + RWym) * dyi2) - fi_p * re * cwz +
+              fi_c * re * cw_m;
+        gu_m = gu;
+        gv_m = gv;
+        cw_m = cwz;
+        tu_m = tu;
+        tv_m = tv;
+        zw_m = zw;
+
+        if (inside) {
+            const size_t g = (size_t)i + (size_t)p.nx * j + sk * k;
+            double xu = alpha * RUc + beta * su, xv = alpha * RVc + beta * sv, xw = alpha * RWc + beta * sw;
+            if (eu) {
+                xu += gamma * __ldg(eu + g);
+                xv += gamma * __ldg(ev + g);
+                xw += gamma * __ldg(ew + g);
+            }
+            ou[g] = xu;
+            ov[g] = xv;
+            ow[g] = (k == p.nz) ? 0.0 : xw;
+        }
+        cp_async_wait<0>(); // plane k + 2
+        const int t = a;
+        a = b;
+        b = free;
+        free = t;
+    }
+}
+
+int launch_adj_rk(const double *u, const double *v, const double *w, const double *ru, const double *rv,
+                  const double *rw, const double *eu, const double *ev, const double *ew, double *ou, double *ov,
+                  double *ow, double alpha, double beta, double gamma, const StepParams &p, const MeshDev &m,
+                  const RkLaunch &l, cudaStream_t st)
+{
+    k_adj_rk<<<l.grid, dim3(AX, AY), sizeof(double) * 3 * ASS, st>>>(u, v, w, ru, rv, rw, eu, ev, ew, ou, ov, ow, alpha,
+                                                                    beta, gamma, p, m, l.kchunk);
+    PL_CHECK_LAUNCH();
+    return 0;
 }
 
 // per-level partial sums of three fields over the degrees of freedom:
@@ -285,10 +386,13 @@ struct AdjWork {
     double *xa = nullptr, *y2 = nullptr, *y1 = nullptr; // adjoint fields (3 fields each)
     double *part = nullptr, *scal = nullptr, *fbar = nullptr;
     size_t nck = 0, nseg = 0; // states that ck and seg hold
+    RkLaunch rk;              // of k_adj_rk
     void release()
     {
         for (double *p : {ck, seg, xa, y2, y1, part}) cudaFree(p);
+        const RkLaunch l = rk;
         *this = AdjWork();
+        rk = l;
     }
     bool reserve(size_t nck_, size_t nseg_, const pl_channel *c)
     {
@@ -355,21 +459,21 @@ int adjoint_step(pl_channel *c, const double *xu, const double *xv, const double
     k_adj_prep<<<adj_grid(p), adj_block(), 0, st>>>(au, av, aw, bu, bv, bw, W.scal, fx, p, c->m);
     PL_CHECK_LAUNCH();
     // P, then W
-    if (launch_calc_rhs_fp64(bu, bv, bw, c->p, p, c->m, st)) return -1;
-    if (ppe_solve_fp64(&c->ppe, c->p, st)) return -1;
+    const int rc = ppe_xfwd_div<double>(&c->ppe, channel_div_in(c, bu, bv, bw), c->p, nullptr, st);
+    if (rc < 0) return -1;
+    if (rc > 0 ? launch_calc_rhs_fp64(bu, bv, bw, c->p, p, c->m, st) || ppe_solve_fp64(&c->ppe, c->p, st)
+               : ppe_solve_fp64_from_x(&c->ppe, c->p, st))
+        return -1;
     k_adj_correct<<<adj_grid(p), adj_block(), 0, st>>>(c->p, bu, bv, bw, p, c->m);
     PL_CHECK_LAUNCH();
     if (level_sums(0, bu, bv, bw, c, W.part, 0.5 * p.dt, 1, W.fbar)) return -1;
     // RK2^T at y1
-    k_adj_rk<<<adj_grid(p), adj_block(), 0, st>>>(c->u1, c->v1, c->w1, bu, bv, bw, nullptr, nullptr, nullptr, cu, cv,
-                                                  cw, 0.5, 0.5 * p.dt, 0.0, p, c->m);
-    PL_CHECK_LAUNCH();
+    if (launch_adj_rk(c->u1, c->v1, c->w1, bu, bv, bw, nullptr, nullptr, nullptr, cu, cv, cw, 0.5, 0.5 * p.dt, 0.0, p,
+                      c->m, W.rk, st))
+        return -1;
     if (level_sums(0, cu, cv, cw, c, W.part, p.dt, 1, W.fbar)) return -1;
     // RK1^T at x
-    k_adj_rk<<<adj_grid(p), adj_block(), 0, st>>>(xu, xv, xw, cu, cv, cw, bu, bv, bw, au, av, aw, 1.0, p.dt, 0.5, p,
-                                                  c->m);
-    PL_CHECK_LAUNCH();
-    return 0;
+    return launch_adj_rk(xu, xv, xw, cu, cv, cw, bu, bv, bw, au, av, aw, 1.0, p.dt, 0.5, p, c->m, W.rk, st);
 }
 
 } // namespace
@@ -429,7 +533,14 @@ extern "C" int pl_adjoint_ke_gradient(pl_channel *c, int nsteps, int every, doub
     cudaStream_t st = c->stream;
     const int nck = (nsteps + every - 1) / every;
     const int nseg = std::min(every, std::max(nsteps, 1));
-    if (!c->adj) c->adj = new AdjWork();
+    if (!c->adj) {
+        RkLaunch l;
+        if (rk_prepare((const void *)k_adj_rk, AT, sizeof(double) * 3 * ASS,
+                       dim3((c->nx + AX - 1) / AX, (c->ny + AY - 1) / AY, 1), c->nz, c->nz, &l))
+            return -1;
+        c->adj = new AdjWork();
+        static_cast<AdjWork *>(c->adj)->rk = l;
+    }
     AdjWork &W = *static_cast<AdjWork *>(c->adj);
     if (!W.reserve(std::max(nck, 1), nseg, c)) {
         W.release();
