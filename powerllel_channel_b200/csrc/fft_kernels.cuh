@@ -101,14 +101,17 @@ __device__ __forceinline__ void pressure_update_staged(const PressureUpdate &pu,
 // (FP64 at N = 384: the forward transform measured faster with 8 columns,
 // 0.173 -> 0.160 ms at 512x384x256, the inverse with 4, 0.177 against 0.182.)
 // Short lines take more columns, so that a stage has work for the 256 threads.
+// Long lines take whole 64-byte row segments at one CTA per SM rather than
+// parts of them at two: FP32 at 1024x768x512, ny = 768, 4 -> 8 columns 1.015
+// -> 0.868 ms forward, 1.026 -> 0.892 ms inverse.
 template <typename V, int N, bool FWD> __host__ __device__ constexpr int pf_y_cols()
 {
-    return N <= 48 ? 32
-                   : (N <= 96 ? 16
-                              : (sizeof(V) == 8 ? ((3072 / N) >= 8 ? 8 : ((3072 / N) >= 4 ? 4 : 2))
-                                                : ((FWD ? 3072 / N : 1536 / N) >= 8
-                                                       ? 8
-                                                       : ((1536 / N) >= 4 ? 4 : ((1536 / N) >= 2 ? 2 : 1)))));
+    constexpr bool fp32 = sizeof(V) == 8;
+    if (N <= 48) return 32;
+    if (N <= 96) return 16;
+    if (N >= 576) return fp32 ? 8 : 4;
+    if (fp32) return 3072 / N >= 8 ? 8 : 4;
+    return (FWD ? 3072 / N : 1536 / N) >= 8 ? 8 : (1536 / N >= 4 ? 4 : 2);
 }
 
 // threads per CTA of the persistent x kernel, and line pairs per group: one
@@ -328,7 +331,8 @@ __global__ void __launch_bounds__(pf_y_threads<T>(),
 // its re-read crosses HBM.  When `part` is given, each group also writes the
 // FP64 sum of its rhs values (in a fixed order) for the plane sums of the
 // mixed path's (0,0) mode.
-constexpr int XDIV_THREADS = 64;
+// one radix-8 butterfly of a stage per thread, up to 128 threads
+template <int N> __host__ __device__ constexpr int xdiv_threads() { return N > 512 ? 128 : 64; }
 
 template <typename T, int N> __host__ __device__ constexpr int xdiv_smem_bytes()
 {
@@ -339,13 +343,13 @@ template <typename T, int N> __host__ __device__ constexpr int xdiv_smem_bytes()
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(XDIV_THREADS) k_xfft_div_pf(DivIn d, T *__restrict__ out,
+__global__ void __launch_bounds__(xdiv_threads<N>()) k_xfft_div_pf(DivIn d, T *__restrict__ out,
                                                               const typename cplx_of<T>::type *__restrict__ twg,
                                                               int ny, int total, double *__restrict__ part)
 {
     pdl_enter();
     using V = typename cplx_of<T>::type;
-    constexpr int NT = XDIV_THREADS, NB = xdiv_lines(N), BUF = (fpad_elems<V>(NB * N) + 1) / 2 * 2;
+    constexpr int NT = xdiv_threads<N>(), NB = xdiv_lines(N), BUF = (fpad_elems<V>(NB * N) + 1) / 2 * 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V *buf = reinterpret_cast<V *>(smem_raw);
     // rows of a group of nb <= NB line pairs: u (2 NB) | v (the row below, 2 NB) | w (2 NB) | w below (2 NB)
@@ -379,6 +383,7 @@ __global__ void __launch_bounds__(XDIV_THREADS) k_xfft_div_pf(DivIn d, T *__rest
         double acc = 0.0;
         auto in = [&](int b, int m) {
             const int mm = (m == 0) ? N - 1 : m - 1;
+            if (NB == 1) b = 0; // known at compile time
             const double *u0 = su + 2 * b * N, *u1 = u0 + N, *vm = sv + 2 * b * N, *v0 = vm + N, *v1 = v0 + N;
             const double *w0 = sw + 2 * b * N, *w1 = w0 + N, *w0m = sm + 2 * b * N, *w1m = w0m + N;
             const double r0 = (u0[m] - u0[mm]) * d.dtidxi + (v0[m] - vm[m]) * d.dtidyi + (w0[m] - w0m[m]) * d.dti * dtidzi_k;
@@ -401,6 +406,7 @@ __global__ void __launch_bounds__(XDIV_THREADS) k_xfft_div_pf(DivIn d, T *__rest
         T *dst = out + (size_t)k * N * ny + (size_t)2 * p * N;
         ct_batch_ip<V, true, false, N, NB, 1, N, NT, 1, ct_nstages(N) - 1>(buf, nb, tw, tid);
         auto put = [&](int b, int m, V A, V Bc) {
+            if (NB == 1) b = 0;
             const V h = split_hc(A, Bc, m, N);
             dst[(size_t)2 * b * N + m] = h.x;
             dst[(size_t)(2 * b + 1) * N + m] = h.y;
@@ -453,7 +459,7 @@ template <typename T, int N> int prepare_x_ct(Ppe *s)
     }
     if (persistent_grid(k_xfft_pf<T, N, true>, x_pf_bytes<T, N>(), groups, NT, &s->grid_x[0]) ||
         persistent_grid(k_xfft_pf<T, N, false>, x_pf_bytes<T, N>(), groups, NT, &s->grid_x[1]) ||
-        persistent_grid(k_xfft_div_pf<T, N>, xdiv_smem_bytes<T, N>(), xdiv_groups<N>(s), XDIV_THREADS, &s->grid_x[3]))
+        persistent_grid(k_xfft_div_pf<T, N>, xdiv_smem_bytes<T, N>(), xdiv_groups<N>(s), xdiv_threads<N>(), &s->grid_x[3]))
         return -1;
     if constexpr (sizeof(T) == 4)
         return persistent_grid(k_xfft_pf<T, N, false, true>, x_pf_bytes<T, N>() + pf_x_pu_bytes<T, N>(), groups, NT,
@@ -516,7 +522,7 @@ template <typename T, int N> int launch_xdiv(Ppe *s, const DivIn &d, T *out, dou
 {
     using V = typename cplx_of<T>::type;
     const V *tw = reinterpret_cast<const V *>(sizeof(T) == 8 ? (const void *)s->d_twx64 : (const void *)s->d_twx32);
-    PL_CUDA_TRY(launch_chained(k_xfft_div_pf<T, N>, s->grid_x[3], XDIV_THREADS, xdiv_smem_bytes<T, N>(), st, d, out, tw,
+    PL_CUDA_TRY(launch_chained(k_xfft_div_pf<T, N>, s->grid_x[3], xdiv_threads<N>(), xdiv_smem_bytes<T, N>(), st, d, out, tw,
                                s->ny, xdiv_groups<N>(s), part));
     return 0;
 }
