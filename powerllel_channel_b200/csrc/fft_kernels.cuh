@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(256) k_xfft_ct(const T *__restrict__ in, size_
     V *tw = buf1 + BUF;
     const int k = blockIdx.y;
     const int p0 = blockIdx.x * NB;
-    const int nb = min(NB, ny / 2 - p0);
+    const int nb = (NB == 1 ? 1 : min(NB, ny / 2 - p0));
     const int tid = threadIdx.x;
     ct_build_twiddles<V, N, 256>(twg, tw, tid);
     for (int e = tid; e < nb * 2 * N; e += 256) {
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(pf_x_threads<T>()) k_xfft_pf(const T *__restri
     ct_build_twiddles<V, N, NT>(twg, tw, tid);
     // PU: the group's rows of q and p (the run the group writes), one commit group
     auto fetch_pu = [&](int g) {
-        const int k = g / gpk, p0 = (g % gpk) * NB, cnt = min(NB, ny / 2 - p0) * 2 * N;
+        const int k = g / gpk, p0 = (g % gpk) * NB, cnt = (NB == 1 ? 1 : min(NB, ny / 2 - p0)) * 2 * N;
         const size_t o = (size_t)k * N * ny + (size_t)2 * p0 * N;
         for (int e = tid * 4; e < cnt; e += NT * 4) {
             if (pu.incremental) cp_async_16(pst + e, pu.q + o + e);
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(pf_x_threads<T>()) k_xfft_pf(const T *__restri
     };
     // rows 2 p0 .. 2 p0 + 2 nb - 1 of plane k are one contiguous run
     auto fetch = [&](int g) {
-        const int k = g / gpk, p0 = (g % gpk) * NB, cnt = min(NB, ny / 2 - p0) * 2 * N;
+        const int k = g / gpk, p0 = (g % gpk) * NB, cnt = (NB == 1 ? 1 : min(NB, ny / 2 - p0)) * 2 * N;
         const T *src = in + (size_t)k * N * ny + (size_t)2 * p0 * N;
         for (int e = tid * CH; e < cnt; e += NT * CH) cp_async_16(stage + e, src + e);
         cp_async_commit();
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(pf_x_threads<T>()) k_xfft_pf(const T *__restri
     if (blockIdx.x < total) fetch(blockIdx.x);
     for (int g = blockIdx.x; g < total; g += gridDim.x) {
         const int tid = opaque_tid();
-        const int k = g / gpk, p0 = (g % gpk) * NB, nb = min(NB, ny / 2 - p0);
+        const int k = g / gpk, p0 = (g % gpk) * NB, nb = (NB == 1 ? 1 : min(NB, ny / 2 - p0));
         cp_async_wait<0>(); // this thread's copies of group g have landed
         __syncthreads();    // ... and everyone's; the previous group is done with buf (and pst)
         if (PU) fetch_pu(g);
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(xdiv_threads<N>()) k_xfft_div_pf(DivIn d, T *_
         for (int e = tid * 2; e < n; e += NT * 2) cp_async_16(dst + e, src + e);
     };
     auto fetch = [&](int g) {
-        const int k = g / gpk, p = (g % gpk) * NB, kg = k + 1, nb = min(NB, ny / 2 - p);
+        const int k = g / gpk, p = (g % gpk) * NB, kg = k + 1, nb = NB == 1 ? 1 : min(NB, ny / 2 - p);
         const size_t r0 = sk * kg + (size_t)2 * p * N;
         copy_rows(su, d.u + r0, 2 * nb * N);
         copy_rows(sv, d.v + sk * kg + (size_t)(p == 0 ? ny - 1 : 2 * p - 1) * N, N);
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(xdiv_threads<N>()) k_xfft_div_pf(DivIn d, T *_
     };
     if (blockIdx.x < total) fetch(blockIdx.x);
     for (int g = blockIdx.x; g < total; g += gridDim.x) {
-        const int k = g / gpk, p = (g % gpk) * NB, nb = min(NB, ny / 2 - p);
+        const int k = g / gpk, p = (g % gpk) * NB, nb = NB == 1 ? 1 : min(NB, ny / 2 - p);
         const double dtidzi_k = __ldg(d.dzf_inv + k + 1);
         cp_async_wait<0>();
         __syncthreads();
