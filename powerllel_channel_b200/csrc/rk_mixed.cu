@@ -27,9 +27,9 @@
 //     the thread's registers from stage 1 of plane k to stage 2 of plane k
 //     (the thread that forms it consumes it), so only u1 goes through
 //     shared memory.
-// 512x384x256: 0.902 -> 0.767 ms (52 % of the measured copy bandwidth at
-// 52 B/point); 256x192x128 0.135 -> 0.098; 1024x768x512 6.21 -> 5.71; 64x64x64
-// 0.041 -> 0.019; 324x162x150, which ran two stage kernels, 0.622 -> 0.20 ms.
+// 512x384x256: 0.902 -> 0.743 ms (54 % of the measured copy bandwidth at
+// 52 B/point); 256x192x128 0.135 -> 0.095; 1024x768x512 6.21 -> 5.24-5.56; 64x64x64
+// 0.041 -> 0.017; 324x162x150, which ran two stage kernels, 0.622 -> 0.168 ms.
 //
 // Stage 2 forms u_hat = u + [ (d1 + d2)/2 - dt G p_pred ] with the bracket in
 // FP32 and the sum in FP64: u, v, w stay FP64, and the projection residual of
@@ -106,8 +106,8 @@ __device__ __forceinline__ f2 w_flux2(const MPlane &P, f2 q, f2 qz)
     return fma2(bc2(P.nrw), sub2(qz, q), mul2(mul2(bc2(0.25f), s), s));
 }
 
-struct MPair { // the fluxes through the bottom faces of a thread's pair
-    f2 fu, fv, fw;
+struct MPair { // a thread's pair: centre values, fluxes through the bottom faces
+    f2 u, v, w, fu, fv, fw;
 };
 
 // the top fluxes of the pair at c (plane k; p: plane k+1)
@@ -119,6 +119,9 @@ __device__ __forceinline__ void top_fluxes2(const float *c, const float *p, cons
     S.fu = top_flux2(P, top_edge2(P, u, uz, add2(w, pk2(w.y, cw[2]))), u, uz);
     S.fv = top_flux2(P, top_edge2(P, v, vz, add2(w, ld2(cw + MW))), v, vz);
     S.fw = w_flux2(P, w, wz);
+    S.u = uz;
+    S.v = vz;
+    S.w = wz;
 }
 
 // x and y parts and the assembly of one component's increment (rk_fused.cu's
@@ -138,13 +141,14 @@ __device__ __forceinline__ f2 assemble2(const MConst &K, f2 sx, f2 sy, f2 q, f2 
 }
 
 // dt * (momentum right-hand side) of the pair at c (plane k; p: plane k+1).
-// S: the fluxes through the bottom faces on entry, the top ones on return.
+// S: on entry the centres of plane k and the fluxes through the bottom faces,
+// on return those of plane k+1.
 template <bool CRF>
 __device__ __forceinline__ void rhs_pair2(const float *c, const float *p, const MPlane &P, const MConst &K, MPair &S,
                                           f2 &du, f2 &dv, f2 &dw)
 {
     const float *cv = c + MPS, *cw = c + 2 * MPS, *pv = p + MPS, *pw = p + 2 * MPS;
-    const f2 u = ld2(c), v = ld2(cv), w = ld2(cw);
+    const f2 u = S.u, v = S.v, w = S.w;
     const f2 uz = ld2(p), vz = ld2(pv), wz = ld2(pw);
     const f2 uS = ld2(c - MW), uN = ld2(c + MW), vS = ld2(cv - MW), vN = ld2(cv + MW), wS = ld2(cw - MW),
              wN = ld2(cw + MW);
@@ -176,6 +180,9 @@ __device__ __forceinline__ void rhs_pair2(const float *c, const float *p, const 
                             sub2(f, S.fw), sub2(wE, wW));
         S.fw = f;
     }
+    S.u = uz;
+    S.v = vz;
+    S.w = wz;
 }
 
 // the same for one point (the stage-1 halo); f: its carried fluxes
@@ -363,7 +370,7 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
             const bool top = p.whi && mq == p.nz; // w1(nz) = 0, the wall
             float *o = sr + a * MSS;
             const float *h0 = ur + b * MSS + hxy0;
-            const f2 cu = ld2(h0), cv = ld2(h0 + MPS), cw = ld2(h0 + 2 * MPS);
+            const f2 cu = s1.u, cv = s1.v, cw = s1.w;
             rhs_pair2<CRF>(h0, ur + a * MSS + hxy0, P, K, s1, d1[0], d1[1], d1[2]);
             if (top) d1[2] = make_float2(-cw.x, -cw.y);
             const f2 nu = add2(cu, d1[0]), nv = add2(cv, d1[1]), nw = add2(cw, d1[2]);
@@ -456,6 +463,9 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
             if (p.wlo && kq == 0) { // w1(0) = 0: no convection through the wall
                 const float *n = sr + a * MSS + hxy0;
                 const f2 u1 = ld2(n), v1 = ld2(n + MPS);
+                s2.u = u1;
+                s2.v = v1;
+                s2.w = ld2(n + 2 * MPS);
                 s2.fu = top_flux2(P, bc2(0.f), sub2(bc2(bcu2), u1), u1);
                 s2.fv = top_flux2(P, bc2(0.f), make_float2(-v1.x, -v1.y), v1);
                 s2.fw = w_flux2(P, bc2(0.f), ld2(n + 2 * MPS));

@@ -1,8 +1,8 @@
-// stencil_rhs.cuh -- the momentum right-hand side of the RK stages, shared by
-// the point-per-thread kernels (stencil.cu) and the fused RK kernel
-// (rk_fused.cu).  Values are fetched through an accessor and neighbour
-// offsets, so the same expressions serve global memory and shared-memory
-// plane rings.
+// stencil_rhs.cuh -- the momentum right-hand side of the RK stages in the
+// reference's expressions, for the point-per-thread kernels (stencil.cu), and
+// the wall fills and reductions that they share with the fused RK kernels.
+// Values are fetched through an accessor, so that the same expressions serve
+// the FP64 fields and the mixed path's sums of a field and an increment.
 #pragma once
 
 #include "stencil.cuh"
@@ -57,11 +57,6 @@ struct LoadSum {
     }
 };
 
-// shared-memory ring offsets fit in 32 bits
-struct Nb32 {
-    int c, xm, xp, ym, yp, zm, zp, xpym, xmyp, xpzm, xmzp, ypzm, ymzp;
-};
-
 // the run and mesh constants of one k-plane of the momentum stencil
 template <typename TC> struct RhsConst {
     TC dx_inv, dy_inv, re_inv, u_crf;
@@ -86,9 +81,8 @@ __device__ __forceinline__ RhsConst<TC> rhs_const(const StepParams &p, const Mes
     return c;
 }
 
-// the momentum right-hand sides with the plane's constants given; CRF false
-// drops the u_crf advection terms (exact when u_crf == 0: they add zero)
-template <typename TC, bool CRF, typename AU, typename AV, typename AW, typename NB>
+// the momentum right-hand sides with the plane's constants given
+template <typename TC, typename AU, typename AV, typename AW, typename NB>
 __device__ __forceinline__ void momentum_rhs_c(const AU &u, const AV &v, const AW &w, const NB &n,
                                                const RhsConst<TC> &cst, TC &ru, TC &rv, TC &rw)
 {
@@ -122,7 +116,7 @@ __device__ __forceinline__ void momentum_rhs_c(const AU &u, const AV &v, const A
     dqt = (uzp - uc) * dzci_k;
     dqb = (uc - uzm) * dzci_km;
     conv = h * ((ue * ue - uw * uw) * dx_inv + (un * vn - us * vs) * dy_inv + (ut * wt - ub * wb) * dzfi_k);
-    if (CRF) conv = conv + half * u_crf * (ue - uw) * dx_inv;
+    conv = conv + half * u_crf * (ue - uw) * dx_inv;
     visc = ((dqe - dqw) * dx_inv + (dqn - dqs) * dy_inv + (dqt - dqb) * dzfi_k) * re_inv;
     ru = visc - conv;
 
@@ -144,7 +138,7 @@ __device__ __forceinline__ void momentum_rhs_c(const AU &u, const AV &v, const A
     dqt = (vzp - vc) * dzci_k;
     dqb = (vc - vzm) * dzci_km;
     conv = h * ((ue * ve - uw * vw) * dx_inv + (vn * vn - vs * vs) * dy_inv + (wt * vt - wb * vb) * dzfi_k);
-    if (CRF) conv = conv + half * u_crf * (ve - vw) * dx_inv;
+    conv = conv + half * u_crf * (ve - vw) * dx_inv;
     visc = ((dqe - dqw) * dx_inv + (dqn - dqs) * dy_inv + (dqt - dqb) * dzfi_k) * re_inv;
     rv = visc - conv;
 
@@ -166,7 +160,7 @@ __device__ __forceinline__ void momentum_rhs_c(const AU &u, const AV &v, const A
     dqt = (wzp - wc) * dzfi_kp;
     dqb = (wc - wzm) * dzfi_k;
     conv = h * ((ue * we - uw * ww) * dx_inv + (vn * wn - vs * ws) * dy_inv + (wt * wt - wb * wb) * dzci_k);
-    if (CRF) conv = conv + half * u_crf * (we - ww) * dx_inv;
+    conv = conv + half * u_crf * (we - ww) * dx_inv;
     visc = ((dqe - dqw) * dx_inv + (dqn - dqs) * dy_inv + (dqt - dqb) * dzci_k) * re_inv;
     rw = visc - conv;
 }
@@ -175,7 +169,7 @@ template <typename TC, typename AU, typename AV, typename AW, typename NB = Nb>
 __device__ __forceinline__ void momentum_rhs(const AU &u, const AV &v, const AW &w, const NB &n, int k,
                                              const StepParams &p, const MeshDev &m, TC &ru, TC &rv, TC &rw)
 {
-    momentum_rhs_c<TC, true>(u, v, w, n, rhs_const<TC>(p, m, k), ru, rv, rw);
+    momentum_rhs_c<TC>(u, v, w, n, rhs_const<TC>(p, m, k), ru, rv, rw);
 }
 
 
