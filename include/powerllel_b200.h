@@ -166,8 +166,7 @@ void *pl_channel_stream(pl_channel *c);
  * 4. Per-phase entries on the channel's device fields (one kernel each,
  *    asynchronous; the step calls them in this order)
  * ====================================================================== */
-int pl_phase_rk(pl_channel *c);         /* both stages in one kernel when nx % 32 == 0 and ny % 8 == 0
-                                           (what pl_channel_step runs), else rk1 then rk2 */
+int pl_phase_rk(pl_channel *c);         /* both stages in one kernel (what pl_channel_step runs) */
 int pl_phase_rk1(pl_channel *c);        /* timeIntVelRK1 + updateBoundVel(u1) */
 int pl_phase_rk2(pl_channel *c);        /* timeIntVelRK2 + updateBoundVel(u) */
 int pl_phase_calc_rhs(pl_channel *c);   /* calcRHS into p */
@@ -200,7 +199,7 @@ int pl_channel_kinetic_energy(pl_channel *c, double *ke);
  * gradient is with respect to the degrees of freedom: u, v on levels 1..nz,
  * w on levels 1..nz-1.  On return u, v, w hold x0 again; p and the stage-1
  * fields are overwritten.  Device memory: (ceil(nsteps/every) + every + 9)
- * fields.  Errors: mixed precision, PDD (trid_parts > 1), nsteps < 0, every < 1. */
+ * fields, kept with the channel until it is destroyed.  Errors: mixed precision, PDD (trid_parts > 1), nsteps < 0, every < 1. */
 int pl_adjoint_ke_gradient(pl_channel *c, int nsteps, int every, double *ke, double *d_gu, double *d_gv,
                            double *d_gw, double grad_f[3]);
 
