@@ -589,11 +589,11 @@ static int phase_rhs_poisson(pl_channel *c)
         const int rc = ppe_xfwd_div<float>(&c->ppe, d, c->r32, c->plane_part, c->stream);
         if (rc < 0) return -1;
         if (rc == 0) {
-            if (launch_plane_sums(c->plane_part, ppe_xdiv_parts(&c->ppe), c->nz, c->mode0, c->stream)) return -1;
             channel_mark(c, "rhs_xfft");
+            const PlaneSums ps{c->plane_part, ppe_xdiv_parts(&c->ppe), c->nz, c->mode0};
             const PressureUpdate pu = mixed_pressure_update(c);
             c->p_stale = true;
-            return ppe_solve_fp32_from_x(&c->ppe, c->r32, c->mode0, c->stream, &pu);
+            return ppe_solve_fp32_from_x(&c->ppe, c->r32, c->mode0, c->stream, &pu, ps);
         }
     } else {
         const int rc = ppe_xfwd_div<double>(&c->ppe, d, c->p, nullptr, c->stream);

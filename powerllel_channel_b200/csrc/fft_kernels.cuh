@@ -254,8 +254,7 @@ template <typename T, int N, bool FWD>
 // 80 bytes at 80; longer lines keep more registers rather than spill
 __global__ void __launch_bounds__(pf_y_threads<T>(),
                                   sizeof(T) == 4 ? (N <= 512 ? 3 : 2) : (N <= 512 ? (FWD ? 2 : 3) : 1))
-    k_yfft_pf(T *__restrict__ data, const typename cplx_of<T>::type *__restrict__ twg,
-                                                 int nx, int total)
+    k_yfft_pf(T *__restrict__ data, const typename cplx_of<T>::type *__restrict__ twg, int nx, int total, PlaneSums ps)
 {
     pdl_enter();
     using V = typename cplx_of<T>::type;
@@ -296,6 +295,24 @@ __global__ void __launch_bounds__(pf_y_threads<T>(),
         cp_async_commit();
     };
     if (blockIdx.x < total) fetch(blockIdx.x);
+    if constexpr (FWD && sizeof(T) == 4) {
+        // plane sums, while the first group's copies are in flight: launch_plane_sums' tree
+        if (ps.part != nullptr) {
+            __shared__ double sh[NT];
+            for (int k = blockIdx.x; k < ps.nz; k += gridDim.x) {
+                double sum = 0.0;
+                for (int b = tid; b < ps.nper; b += NT) sum += __ldg(ps.part + (size_t)k * ps.nper + b);
+                sh[tid] = sum;
+                __syncthreads();
+                for (int o = NT / 2; o > 0; o >>= 1) {
+                    if (tid < o) sh[tid] += sh[tid + o];
+                    __syncthreads();
+                }
+                if (tid == 0) ps.out[k] = sh[0];
+                __syncthreads();
+            }
+        }
+    }
     for (int g = blockIdx.x; g < total; g += gridDim.x) {
         const int k = g / gpk, c0 = (g % gpk) * W, nb = min(W, ncol - c0);
         V *plane = reinterpret_cast<V *>(data) + (size_t)k * N * ncol;
@@ -509,12 +526,12 @@ int launch_x_ct(const Ppe *s, const T *in, size_t in_off, size_t in_sj, size_t i
     return 0;
 }
 
-template <typename T, int N, bool FWD> int launch_y_ct(const Ppe *s, T *data, cudaStream_t st)
+template <typename T, int N, bool FWD> int launch_y_ct(const Ppe *s, T *data, cudaStream_t st, const PlaneSums &ps)
 {
     using V = typename cplx_of<T>::type;
     const V *tw = reinterpret_cast<const V *>(sizeof(T) == 8 ? (const void *)s->d_twy64 : (const void *)s->d_twy32);
     PL_CUDA_TRY(launch_chained(k_yfft_pf<T, N, FWD>, s->grid_y[FWD ? 0 : 1], pf_y_threads<T>(), y_pf_bytes<T, N, FWD>(),
-                               st, data, tw, s->nx, y_pf_groups<T, N, FWD>(s)));
+                               st, data, tw, s->nx, y_pf_groups<T, N, FWD>(s), ps));
     return 0;
 }
 
@@ -534,8 +551,8 @@ template <typename T, int N> int launch_xdiv(Ppe *s, const DivIn &d, T *out, dou
                                          T, cudaStream_t, const PressureUpdate *, bool *);                             \
     template int launch_x_ct<T, n, false>(const Ppe *, const T *, size_t, size_t, size_t, T *, size_t, size_t, size_t, \
                                           T, cudaStream_t, const PressureUpdate *, bool *);                            \
-    template int launch_y_ct<T, n, true>(const Ppe *, T *, cudaStream_t);                                              \
-    template int launch_y_ct<T, n, false>(const Ppe *, T *, cudaStream_t);                                             \
+    template int launch_y_ct<T, n, true>(const Ppe *, T *, cudaStream_t, const PlaneSums &);                           \
+    template int launch_y_ct<T, n, false>(const Ppe *, T *, cudaStream_t, const PlaneSums &);                          \
     template int launch_xdiv<T, n>(Ppe *, const DivIn &, T *, double *, cudaStream_t);
 #define PL_FFT_INSTANTIATE(n) PL_FFT_INSTANTIATE_T(double, n) PL_FFT_INSTANTIATE_T(float, n)
 

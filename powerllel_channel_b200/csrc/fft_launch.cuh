@@ -35,8 +35,8 @@ template <typename T, int N> int prepare_y_ct(Ppe *s);
 template <typename T, int N, bool FWD>
 int launch_x_ct(const Ppe *s, const T *in, size_t in_off, size_t in_sj, size_t in_sk, T *out, size_t out_off,
                 size_t out_sj, size_t out_sk, T scale, cudaStream_t st, const PressureUpdate *pu, bool *fused);
-// y transform, in place
-template <typename T, int N, bool FWD> int launch_y_ct(const Ppe *s, T *data, cudaStream_t st);
+// y transform, in place (ps: the plane sums that a forward one forms as well)
+template <typename T, int N, bool FWD> int launch_y_ct(const Ppe *s, T *data, cudaStream_t st, const PlaneSums &ps);
 // calcRHS and the forward x transform
 template <typename T, int N> int launch_xdiv(Ppe *s, const DivIn &d, T *out, double *part, cudaStream_t st);
 

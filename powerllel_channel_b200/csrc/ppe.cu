@@ -22,6 +22,7 @@
 
 #include "fft_launch.cuh"
 #include "ppe.cuh"
+#include "stencil.cuh" // launch_plane_sums
 #include "tmem.cuh"
 #include "trid_tables.h"
 
@@ -1658,20 +1659,23 @@ static int launch_x(const Ppe *s, bool fwd, const T *in, size_t in_off, size_t i
     return pu ? launch_pressure_update(s, out, pu, st) : 0;
 }
 
-template <typename T> static int launch_y(const Ppe *s, bool fwd, T *data, cudaStream_t st)
+// ps: plane sums that the kernels consuming the forward transform need as well
+template <typename T>
+static int launch_y(const Ppe *s, bool fwd, T *data, cudaStream_t st, const PlaneSums &ps = PlaneSums{})
 {
     using V = typename cplx_of<T>::type;
     switch (s->ny) {
 #define PL_Y_CASE(n)                                                                                               \
     case n:                                                                                                        \
         if ((uintptr_t)data % 16 == 0)                                                                             \
-            return fwd ? launch_y_ct<T, n, true>(s, data, st) : launch_y_ct<T, n, false>(s, data, st);             \
+            return fwd ? launch_y_ct<T, n, true>(s, data, st, ps) : launch_y_ct<T, n, false>(s, data, st, ps);             \
         break;
         PL_FFT_CT_SIZES(PL_Y_CASE)
 #undef PL_Y_CASE
     default:
         break;
     }
+    if (ps.part && launch_plane_sums(ps.part, ps.nper, ps.nz, ps.out, st)) return -1;
     const int w = y_cols_per_cta(s->nx, s->ny);
     dim3 grid((s->nx / 2 + w - 1) / w, s->nz);
     const size_t shm = 2 * sizeof(V) * (size_t)fpad_elems<V>(w * s->ny);
@@ -1860,10 +1864,11 @@ int ppe_solve_fp32(Ppe *s, float *d_var, const double *mode0, cudaStream_t st, c
     return ppe_solve_fp32_from_x(s, d_var, mode0, st, pu);
 }
 
-int ppe_solve_fp32_from_x(Ppe *s, float *d_var, const double *mode0, cudaStream_t st, const PressureUpdate *pu)
+int ppe_solve_fp32_from_x(Ppe *s, float *d_var, const double *mode0, cudaStream_t st, const PressureUpdate *pu,
+                          const PlaneSums &ps)
 {
     const size_t nxl = s->nx, nxy = (size_t)s->nx * s->ny;
-    if (launch_y<float>(s, true, d_var, st)) return -1;
+    if (launch_y<float>(s, true, d_var, st, ps)) return -1;
     mark(s, "ppe_yfft_fwd");
     if (launch_trid<float>(s, d_var, st, mode0)) return -1;
     mark(s, s->nparts ? "ppe_pdd" : "ppe_thomas");

@@ -107,6 +107,14 @@ struct DivIn {
 // not apply: nx not a compile-time transform length.
 template <typename T> int ppe_xfwd_div(Ppe *s, const DivIn &d, T *out, double *part, cudaStream_t st);
 int ppe_xdiv_parts(const Ppe *s); // partial sums per plane that ppe_xfwd_div writes
+// out[k] = the sum over the nper partials of plane k, in a fixed order (the
+// mixed path's (0,0) right-hand side): formed by the forward y transform, as
+// a kernel of its own it was a launch and 3 us of every step
+struct PlaneSums {
+    const double *part = nullptr; // null: none asked for
+    int nper = 0, nz = 0;
+    double *out = nullptr;
+};
 // FP64 solve when d_var already holds the forward x transform
 int ppe_solve_fp64_from_x(Ppe *s, double *d_var, cudaStream_t st);
 
@@ -117,8 +125,9 @@ struct PressureUpdate {
 };
 int ppe_solve_fp32(Ppe *s, float *d_var, const double *mode0, cudaStream_t st, const PressureUpdate *pu = nullptr);
 // the same solve when d_var already holds the forward x transform
+// (ps: the partial sums that mode0 is to hold the plane sums of)
 int ppe_solve_fp32_from_x(Ppe *s, float *d_var, const double *mode0, cudaStream_t st,
-                          const PressureUpdate *pu = nullptr);
+                          const PressureUpdate *pu = nullptr, const PlaneSums &ps = PlaneSums{});
 
 // the plan of z slab `rank` of `nranks` (nz_global planes distributed as
 // decomp_2d.c:261-283 distributes them; PDD across the slabs)
