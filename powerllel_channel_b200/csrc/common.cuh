@@ -44,9 +44,9 @@ const char *get_error();
         }                                                                                  \
     } while (0)
 
-// Launch of a kernel that begins with pdl_enter(): its CTAs may be scheduled
-// while the stream's previous kernel drains, and wait there for its results.
-// The step is a chain of eight short kernels, whose launch latencies add up on
+// Launch of a kernel that begins with pdl_enter(): its launch is prepared while
+// the stream's previous kernel runs, and its CTAs start as that one's end.  The
+// step is a chain of seven short kernels, whose launch latencies add up on
 // small grids.
 template <typename... K, typename... A>
 inline cudaError_t launch_chained(void (*kern)(K...), dim3 grid, dim3 block, size_t shm, cudaStream_t st, A &&...args)
@@ -66,12 +66,16 @@ inline cudaError_t launch_chained(void (*kern)(K...), dim3 grid, dim3 block, siz
 
 // First statement of such a kernel: waits until the previous kernel of the
 // stream has completed and its writes are visible (it waited for its own
-// predecessor in turn), then lets the next one's CTAs be scheduled.  Without
-// the launch attribute both are no-ops.
+// predecessor in turn).  Without the launch attribute it is a no-op.  The next
+// kernel is released by this one's end: releasing it here as well
+// (griddepcontrol.launch_dependents) let its waiting CTAs take the room and
+// the shared-memory split that the running kernel's own tail needs, and cost
+// more than the launches it hid (step back to back, us: plain launches 50.4,
+// wait alone 36.8, early release 42.8 at 64x64x64; 334, 316 and 350 at
+// 256x192x128 PDD-4; 2435, 2428 and 2592 at 512x384x256, all FP64).
 __device__ __forceinline__ void pdl_enter()
 {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
 template <typename T> struct cplx_of;
