@@ -66,6 +66,14 @@ def test_pdd_by_partition_size(gpu, oracle_mod, nz, nparts, precision, tol):
     assert np.abs(got - ref).max() < tol * np.abs(ref).max()
 
 
+def test_pdd_on_an_array_larger_than_l2(gpu, oracle_mod):
+    """151 MB in partitions of 24 rows: batches of 8 rows whose successors are requested into L2."""
+    plb, O = gpu, oracle_mod
+    g, r, ref = rhs_and_reference(O, 512, 384, 96, 4)
+    got = solve(plb, g, r, plb.PL_FP64, 4)
+    assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("nx,ny,nz", [(16, 6, 4), (54, 18, 14), (96, 24, 22), (162, 16, 10), (324, 8, 6)])
 def test_step_matches_phases(gpu, precision, nx, ny, nz):
