@@ -1111,7 +1111,7 @@ __global__ void __launch_bounds__(1024) k_pdd_par(const T *xin, double *xs, T *x
 constexpr int PTM_G = 8;
 constexpr size_t L2_BYTES = (size_t)126 << 20;
 
-__host__ __device__ constexpr int pdd_tm_static_smem() { return 2 * 8 * 32 * 8 + 16; }
+__host__ __device__ constexpr int pdd_tm_static_smem(int nc) { return nc * 2 * 8 * 32 * 8 + 16; }
 
 __device__ __forceinline__ void prefetch_l2(const void *q) { asm volatile("prefetch.global.L2 [%0];" ::"l"(q)); }
 
@@ -1119,65 +1119,94 @@ __device__ __forceinline__ void prefetch_l2(const void *q) { asm volatile("prefe
 // where the arrays do not stay in L2 anyway: 1024x768x512, 8 partitions, 2.81 ->
 // 2.55 ms mixed, 3.25 -> 2.85 FP64; 256x192x128, 4 partitions (a 25 or 50 MB
 // array), 38.7 -> 38.8 and 37.3 -> 39.3 us.
-template <typename T, int B, bool PF>
+// NC: columns per thread.  Two are the mirror rows py and ny - py, which have
+// one eigenvalue class: each class-table entry is loaded once for both, and
+// the two recurrences interleave.  The tables are 32 of the 40 bytes that a
+// mixed row takes through L2, and their loads stall it.  1024x768x512, P 8:
+// 2.47 -> 2.03 ms mixed, 2.71 -> 2.51 FP64; 256x192x128, P 4: 38.8 -> 30.9 and
+// 38.0 -> 33.0 us.  Batches of 8 rows (128 registers instead of 164) were
+// slower: 2.14 ms and 40.9 us mixed.
+template <typename T, int B, bool PF, int NC>
 __global__ void __launch_bounds__(256) k_pdd_tm(const T *xin, T *xout, TridDev t, PddDev p, const double *mode0,
                                                 int kmax, uint32_t tcols)
 {
     pdl_enter();
     constexpr int G = PTM_G, H = B / G;
-    __shared__ double edge[2][8][32]; // [first / last local value][partition][column]
+    using X = typename std::conditional<NC == 1, double, T>::type; // two columns: converted at use, fewer registers
+    __shared__ double edge[2][8][NC][32]; // [first / last local value][partition][column]
     __shared__ uint32_t tslot;
     const int cx = threadIdx.x, m = threadIdx.y;
-    const int q = blockIdx.x * 32 + cx, ncol = t.nx * t.ny;
-    const bool valid = q < ncol;
-    const int qq = valid ? q : 0, px = qq % t.nx, py = trid_pair_row(qq / t.nx, t.ny);
-    const size_t col = (size_t)px + (size_t)t.nx * py, stride = (size_t)t.nx * t.ny;
-    const size_t cls = trid_class(px, py, t), cstride = (size_t)t.ncx * t.ncy;
+    const int q = blockIdx.x * 32 + cx, nrow = NC == 2 ? t.ny / 2 + 1 : t.ny;
+    const int b = q / t.nx, px = q - b * t.nx;
+    bool valid[NC];
+    size_t col[NC];
+    valid[0] = b < nrow;
+    const int py = NC == 2 ? b : trid_pair_row(b, t.ny);
+    col[0] = valid[0] ? (size_t)px + (size_t)t.nx * py : 0;
+    if (NC == 2) { // the mirror row; rows 0 and ny / 2 have none
+        valid[NC - 1] = valid[0] && b > 0 && 2 * b != t.ny;
+        col[NC - 1] = valid[NC - 1] ? (size_t)px + (size_t)t.nx * (t.ny - b) : col[0];
+    }
+    const size_t stride = (size_t)t.nx * t.ny;
+    const size_t cls = valid[0] ? trid_class(px, py, t) : 0, cstride = (size_t)t.ncx * t.ncy;
     const int k0 = p.kst[m], ke = p.ksz[m], ng = ke / B;
-    const bool z = mode0 != nullptr && valid && col == 0; // mixed path: the (0,0) column from the plane sums
+    const bool z = mode0 != nullptr && valid[0] && col[0] == 0; // mixed path: the (0,0) column from the plane sums
 
     if (m == 0) tmem_alloc(&tslot, tcols);
     tmem_fence_before_sync();
     __syncthreads();
     tmem_fence_after_sync();
-    const uint32_t tb = tslot + ((uint32_t)((m & 3) * 32) << 16) + (uint32_t)((m >> 2) * 2 * kmax);
+    const uint32_t tb = tslot + ((uint32_t)((m & 3) * 32) << 16) + (uint32_t)((m >> 2) * NC * 2 * kmax);
 
     // forward elimination of the partition (ssolve_trid :319-330; the
     // multiplier is 0 at its first row)
-    double xp = 0.0;
+    double xp[NC];
+#pragma unroll
+    for (int n = 0; n < NC; n++) xp[n] = 0.0;
     for (int g = 0; g < ng; g++) {
-        double xv[B], mv[B];
+        X xv[NC][B];
+        double mv[B];
 #pragma unroll
         for (int u = 0; u < B; u++) {
             const int k = k0 + g * B + u;
-            xv[u] = z ? mode0[k] : (double)xin[col + (size_t)k * stride];
+#pragma unroll
+            for (int n = 0; n < NC; n++) xv[n][u] = (X)xin[col[n] + (size_t)k * stride];
             mv[u] = __ldg(t.mult + cls + (size_t)k * cstride);
         }
         if (PF && g + 1 < ng) { // the next batch on its way to L2
 #pragma unroll
             for (int u = 0; u < B; u++) {
                 const int kn = k0 + (g + 1) * B + u;
-                prefetch_l2(xin + col + (size_t)kn * stride);
+#pragma unroll
+                for (int n = 0; n < NC; n++) prefetch_l2(xin + col[n] + (size_t)kn * stride);
                 prefetch_l2(t.mult + cls + (size_t)kn * cstride);
             }
         }
 #pragma unroll
         for (int h = 0; h < H; h++) {
-            uint32_t v[2 * G];
+            uint32_t v[NC][2 * G];
 #pragma unroll
             for (int u = 0; u < G; u++) {
-                xp = xv[h * G + u] - mv[h * G + u] * xp;
-                v[2 * u] = (uint32_t)__double2loint(xp);
-                v[2 * u + 1] = (uint32_t)__double2hiint(xp);
+#pragma unroll
+                for (int n = 0; n < NC; n++) {
+                    double x = (double)xv[n][h * G + u];
+                    if (sizeof(T) == 4 && n == 0 && z) x = mode0[k0 + g * B + h * G + u];
+                    xp[n] = x - mv[h * G + u] * xp[n];
+                    v[n][2 * u] = (uint32_t)__double2loint(xp[n]);
+                    v[n][2 * u + 1] = (uint32_t)__double2hiint(xp[n]);
+                }
             }
             __syncwarp();
-            tmem_st16(tb + 2 * (g * B + h * G), v);
+#pragma unroll
+            for (int n = 0; n < NC; n++) tmem_st16(tb + 2 * (n * kmax + g * B + h * G), v[n]);
         }
     }
     tmem_wait_st();
     // back substitution (:332-356): x = (x - c x_{k+1}) / b, with x_{k+1} = 0
     // above the partition's last row; the local solution replaces the swept rows
-    double w = 0.0, first = 0.0, last = 0.0;
+    double w[NC], last[NC];
+#pragma unroll
+    for (int n = 0; n < NC; n++) w[n] = last[n] = 0.0;
     for (int g = ng - 1; g >= 0; g--) {
         double rv[B];
 #pragma unroll
@@ -1188,47 +1217,59 @@ __global__ void __launch_bounds__(256) k_pdd_tm(const T *xin, T *xout, TridDev t
         }
 #pragma unroll
         for (int h = H - 1; h >= 0; h--) {
-            uint32_t v[2 * G];
+            uint32_t v[NC][2 * G];
             __syncwarp();
-            tmem_ld16_start(tb + 2 * (g * B + h * G), v);
+#pragma unroll
+            for (int n = 0; n < NC; n++) tmem_ld16_start(tb + 2 * (n * kmax + g * B + h * G), v[n]);
             double cv[G];
 #pragma unroll
             for (int u = 0; u < G; u++) cv[u] = __ldg(t.c + k0 + g * B + h * G + u);
-            tmem_wait_ld(v);
+#pragma unroll
+            for (int n = 0; n < NC; n++) tmem_wait_ld(v[n]);
 #pragma unroll
             for (int u = G - 1; u >= 0; u--) {
-                const double s = __hiloint2double((int)v[2 * u + 1], (int)v[2 * u]);
-                w = (s - cv[u] * w) * rv[h * G + u];
-                if (g == ng - 1 && h == H - 1 && u == G - 1) last = w;
-                v[2 * u] = (uint32_t)__double2loint(w);
-                v[2 * u + 1] = (uint32_t)__double2hiint(w);
+#pragma unroll
+                for (int n = 0; n < NC; n++) {
+                    const double s = __hiloint2double((int)v[n][2 * u + 1], (int)v[n][2 * u]);
+                    w[n] = (s - cv[u] * w[n]) * rv[h * G + u];
+                    if (g == ng - 1 && h == H - 1 && u == G - 1) last[n] = w[n];
+                    v[n][2 * u] = (uint32_t)__double2loint(w[n]);
+                    v[n][2 * u + 1] = (uint32_t)__double2hiint(w[n]);
+                }
             }
             __syncwarp();
-            tmem_st16(tb + 2 * (g * B + h * G), v);
+#pragma unroll
+            for (int n = 0; n < NC; n++) tmem_st16(tb + 2 * (n * kmax + g * B + h * G), v[n]);
         }
     }
-    first = w;
     tmem_wait_st();
-    edge[0][m][cx] = first;
-    edge[1][m][cx] = last;
+#pragma unroll
+    for (int n = 0; n < NC; n++) {
+        edge[0][m][n][cx] = w[n];
+        edge[1][m][n][cx] = last[n];
+    }
     __syncthreads();
     // the truncated 2x2 systems at the partition's two interfaces (:423-438)
-    auto iface = [&](int mm, double &y2, double &y3) {
+    auto iface = [&](int mm, int n, double &y2, double &y3) {
         const int kt = p.kst[mm] + p.ksz[mm] - 1;
         const double wt = __ldg(p.w + cls + (size_t)kt * cstride);
         const double tv = __ldg(p.tmpv + cls + (size_t)mm * cstride);
-        const double xt = edge[1][mm][cx], tvar = edge[0][mm + 1][cx];
+        const double xt = edge[1][mm][n][cx], tvar = edge[0][mm + 1][n][cx];
         const double det = wt * tv - 1.0;
         y2 = (xt * tv - tvar) / det;
         y3 = (tvar * wt - xt) / det;
-        if (pdd_gauge00(mode0, col, p.nparts)) {
+        if (pdd_gauge00(mode0, col[n], p.nparts)) {
             y2 = tvar;
             y3 = 0.0;
         }
     };
-    double y1 = 0.0, y2 = 0.0, unused;
-    if (m > 0) iface(m - 1, unused, y1);
-    if (m + 1 < p.nparts) iface(m, y2, unused);
+    double y1[NC], y2[NC], unused;
+#pragma unroll
+    for (int n = 0; n < NC; n++) {
+        y1[n] = y2[n] = 0.0;
+        if (m > 0) iface(m - 1, n, unused, y1[n]);
+        if (m + 1 < p.nparts) iface(m, n, y2[n], unused);
+    }
     // correction x = x_local - v y1 - w y2 (:452-464)
     for (int g = 0; g < ng; g++) {
         double vv[B], wv[B];
@@ -1248,16 +1289,21 @@ __global__ void __launch_bounds__(256) k_pdd_tm(const T *xin, T *xout, TridDev t
         }
 #pragma unroll
         for (int h = 0; h < H; h++) {
-            uint32_t v[2 * G];
+            uint32_t v[NC][2 * G];
             __syncwarp();
-            tmem_ld16_start(tb + 2 * (g * B + h * G), v);
-            tmem_wait_ld(v);
-            if (valid) {
 #pragma unroll
-                for (int u = 0; u < G; u++) {
-                    const double x = __hiloint2double((int)v[2 * u + 1], (int)v[2 * u]);
-                    xout[col + (size_t)(k0 + g * B + h * G + u) * stride] =
-                        (T)(x - vv[h * G + u] * y1 - wv[h * G + u] * y2);
+            for (int n = 0; n < NC; n++) tmem_ld16_start(tb + 2 * (n * kmax + g * B + h * G), v[n]);
+#pragma unroll
+            for (int n = 0; n < NC; n++) tmem_wait_ld(v[n]);
+#pragma unroll
+            for (int n = 0; n < NC; n++) {
+                if (valid[n]) {
+#pragma unroll
+                    for (int u = 0; u < G; u++) {
+                        const double x = __hiloint2double((int)v[n][2 * u + 1], (int)v[n][2 * u]);
+                        xout[col[n] + (size_t)(k0 + g * B + h * G + u) * stride] =
+                            (T)(x - vv[h * G + u] * y1[n] - wv[h * G + u] * y2[n]);
+                    }
                 }
             }
         }
@@ -1786,21 +1832,32 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
         p.w = s->d_w;
         p.tmpv = s->d_tmpv;
         const int ncol = s->nx * s->ny;
-        const int cells = ((s->nparts + 3) / 4) * 2 * kmax; // TMEM columns of one CTA
+        const int cells = ((s->nparts + 3) / 4) * 2 * kmax; // TMEM columns of one CTA and column per thread
         if (groups && s->nparts <= 8 && cells <= 512) {
             // partitions in tensor memory; the dynamic shared memory (unused)
             // caps the CTAs on an SM at what its 512 TMEM columns hold
             uint32_t tcols = 32;
-            while (tcols < (uint32_t)cells) tcols *= 2;
-            const int per_sm = std::max(1, std::min(512 / (int)tcols, 2048 / (32 * s->nparts)));
-            const int dyn = std::max(0, 233472 / per_sm - 1024 - pdd_tm_static_smem() - 512);
-            // loads of 16 rows in flight where the partitions allow, else 8
+            // Two mirrored columns per thread where their CTAs fill the chip,
+            // except for 5 to 8 short partitions (64 .. 256 cells: one CTA of
+            // 256 threads per SM by its registers) on arrays that stay in L2
+            // (one column against two per thread, us, mixed: 256x192x128 P 4
+            // 38.8, 30.9; 512x384x256 P 8 390, 267, P 4 326, 255; 64x64x64 P 4
+            // 9.9, 10.4 on 66 CTAs; 256x192x256 P 8 75.6, 79.4).
             const bool pf = sizeof(T) * (size_t)ncol * s->nz > L2_BYTES;
-            auto kern = groups2 ? (pf ? k_pdd_tm<T, 2 * PTM_G, true> : k_pdd_tm<T, 2 * PTM_G, false>)
-                                : (pf ? k_pdd_tm<T, PTM_G, true> : k_pdd_tm<T, PTM_G, false>);
-            if (dyn > 48 * 1024)
+            const int pairs = s->nx * (s->ny / 2 + 1);
+            const int nc = groups2 && 2 * cells <= 512 && pairs >= 32 * 148 &&
+                                   (pf || s->nparts <= 4 || 2 * cells > 256) ? 2 : 1;
+            while (tcols < (uint32_t)(nc * cells)) tcols *= 2;
+            const int per_sm = std::max(1, std::min(512 / (int)tcols, 2048 / (32 * s->nparts)));
+            const int dyn = std::max(0, 233472 / per_sm - 1024 - pdd_tm_static_smem(nc) - 512);
+            // loads of 16 rows in flight where the partitions allow, else 8
+            auto kern = nc == 2 ? (pf ? k_pdd_tm<T, 2 * PTM_G, true, 2> : k_pdd_tm<T, 2 * PTM_G, false, 2>)
+                        : groups2 ? (pf ? k_pdd_tm<T, 2 * PTM_G, true, 1> : k_pdd_tm<T, 2 * PTM_G, false, 1>)
+                                  : (pf ? k_pdd_tm<T, PTM_G, true, 1> : k_pdd_tm<T, PTM_G, false, 1>);
+            const int cols = nc == 2 ? pairs : ncol; // threads per partition
+            if (dyn + pdd_tm_static_smem(nc) > 48 * 1024)
                 PL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-            PL_CUDA_TRY(launch_chained(kern, (ncol + 31) / 32, dim3(32, s->nparts), dyn, st, x, x, t, p, sizeof(T) == 4 ? mode0 : nullptr, kmax, tcols));
+            PL_CUDA_TRY(launch_chained(kern, (cols + 31) / 32, dim3(32, s->nparts), dyn, st, x, x, t, p, sizeof(T) == 4 ? mode0 : nullptr, kmax, tcols));
         } else {
             PL_CUDA_TRY(launch_chained(k_pdd_par<T>, (ncol + 31) / 32, dim3(32, s->nparts), 0, st, x, s->d_scratch, x, t, p, sizeof(T) == 4 ? mode0 : nullptr));
         }

@@ -74,6 +74,17 @@ def test_pdd_on_an_array_larger_than_l2(gpu, oracle_mod):
     assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("nx,ny,nz,nparts", [(162, 64, 48, 3), (128, 72, 64, 4), (16, 648, 48, 3), (216, 96, 384, 8)])
+def test_pdd_two_columns_per_thread(gpu, oracle_mod, nx, ny, nz, nparts, precision, tol):
+    """At least 148 CTAs of mirrored column pairs: a ragged last CTA, the rows without a mirror (0 and
+    ny / 2), exactly 148, and partitions whose pairs take 384 of the 512 cells."""
+    plb, O = gpu, oracle_mod
+    g, r, ref = rhs_and_reference(O, nx, ny, nz, nparts)
+    got = solve(plb, g, r, plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED, nparts)
+    assert np.abs(got - ref).max() < tol * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("nx,ny,nz", [(16, 6, 4), (54, 18, 14), (96, 24, 22), (162, 16, 10), (324, 8, 6)])
 def test_step_matches_phases(gpu, precision, nx, ny, nz):
