@@ -29,10 +29,11 @@
 //     shared memory.
 // 512x384x256: 0.902 -> 0.743 ms (54 % of the measured copy bandwidth at
 // 52 B/point); 256x192x128 0.135 -> 0.095; 1024x768x512 6.21 -> 5.24-5.56; 64x64x64
-// 0.041 -> 0.017; 324x162x150, which ran two stage kernels, 0.622 -> 0.168 ms.
+// 0.041 -> 0.017; 324x162x150, which ran two stage kernels, 0.622 -> 0.223 ms
+// (WIDE below).
 //
 // Stage 2 forms u_hat = u + [ (d1 + d2)/2 - dt G p_pred ] with the bracket in
-// FP32 and the sum in FP64: u, v, w stay FP64, and the projection residual of
+// FP32 (WIDE: in FP64) and the sum in FP64: u, v, w stay FP64, and the projection residual of
 // the increment solve is the FP64 divergence of the stored u_hat, whatever
 // rounding the bracket carries.
 #include <type_traits>
@@ -232,7 +233,12 @@ __device__ __forceinline__ void rhs_one(const float *c, const float *p, const MP
 
 } // namespace
 
-template <bool CRF>
+// WIDE: the stage-1 field and stage 2's update are formed in FP64, from the
+// FP64 fields and the FP32 increments, as the stage kernels (stencil.cu) form
+// them: u1 = (float)(u + d1), u_hat = ((u + d1) + d2 + u) / 2 - dt G p_pred.
+// Otherwise u1 = (float)u + d1 and the bracket are FP32, where stage 2 sees the
+// rounding of u that stage 1 saw and another one.
+template <bool CRF, bool WIDE>
 __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u, const double *__restrict__ v,
                                                    const double *__restrict__ w, double *__restrict__ uo,
                                                    double *__restrict__ vo, double *__restrict__ wo, StepParams p,
@@ -318,6 +324,9 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
     const bool inside = gi < p.nx && gj < p.ny;
     const size_t gA = (size_t)gi + (size_t)p.nx * gj;
     const size_t gE = gi == p.nx - 2 ? gA - gi : gA + 2, gN = gj == p.ny - 1 ? gi : gA + p.nx;
+    // WIDE: where the FP64 values of the thread's pair and rim point are (wrapped)
+    const int swA = WIDE ? gj % p.ny * p.nx + gi % p.nx : 0;
+    const int swH = WIDE ? (j0 - 2 + hxy1 / MW + p.ny) % p.ny * p.nx + (i0 - 2 + hxy1 % MW + p.nx) % p.nx : 0;
 
     issue(mstart - 1);
     for (int k = mstart - 1 + tid; k <= mend; k += MT) {
@@ -352,9 +361,20 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
     // d1 of the own pair at the planes mq and mq - 1; the prediction at stage
     // 2's next plane
     f2 d1[3] = {}, e1[3] = {};
+    // WIDE: the pair's FP64 values at those planes, loaded once for both stages
+    // (loading them for each: 0.237 against 0.223 ms at 324x162x150)
+    double2 q1[3] = {}, e64[3] = {};
     f2 qc = bc2(0.f);
     double su = 0.0;
-    const float bcu2 = (float)(2.0 * (0.0 - p.u_crf));
+    const double b2 = 2.0 * (0.0 - p.u_crf); // imposeNoSlipBC's image
+    const float bcu2 = (float)b2;
+    float eh = 0.f; // WIDE: the rim point's stage-1 increment of u
+    // FP64 value and increment, rounded once
+    auto sum32 = [](double2 q, f2 d) { return make_float2((float)(q.x + (double)d.x), (float)(q.y + (double)d.y)); };
+    auto image32 = [&](double2 q, f2 d) {
+        return make_float2((float)((b2 - q.x) - (double)d.x), (float)((b2 - q.y) - (double)d.y));
+    };
+    auto pair64 = [&](const double *f, size_t at) { return __ldg(reinterpret_cast<const double2 *>(f + at)); };
 
     // one plane of the march: PH = (mq - mstart) % 2
     auto march = [&](auto PH, int mq) {
@@ -370,10 +390,32 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
             const bool top = p.whi && mq == p.nz; // w1(nz) = 0, the wall
             float *o = sr + a * MSS;
             const float *h0 = ur + b * MSS + hxy0;
-            const f2 cu = s1.u, cv = s1.v, cw = s1.w;
+            [[maybe_unused]] const f2 cu = s1.u, cv = s1.v;
+            const f2 cw = s1.w;
+            [[maybe_unused]] double h64[3] = {0.0, 0.0, 0.0};
+            if constexpr (WIDE) {
+                const size_t at = sk * mq + swA, ah = sk * mq + swH;
+                q1[0] = pair64(u, at);
+                q1[1] = pair64(v, at);
+                q1[2] = pair64(w, at);
+                if (hval) {
+                    h64[0] = __ldg(u + ah);
+                    h64[1] = __ldg(v + ah);
+                    h64[2] = __ldg(w + ah);
+                }
+            }
             rhs_pair2<CRF>(h0, ur + a * MSS + hxy0, P, K, s1, d1[0], d1[1], d1[2]);
             if (top) d1[2] = make_float2(-cw.x, -cw.y);
-            const f2 nu = add2(cu, d1[0]), nv = add2(cv, d1[1]), nw = add2(cw, d1[2]);
+            f2 nu, nv, nw;
+            if constexpr (WIDE) {
+                nu = sum32(q1[0], d1[0]);
+                nv = sum32(q1[1], d1[1]);
+                nw = top ? bc2(0.f) : sum32(q1[2], d1[2]);
+            } else {
+                nu = add2(cu, d1[0]);
+                nv = add2(cv, d1[1]);
+                nw = add2(cw, d1[2]);
+            }
             *reinterpret_cast<float2 *>(o + hxy0) = nu;
             *reinterpret_cast<float2 *>(o + hxy0 + MPS) = nv;
             *reinterpret_cast<float2 *>(o + hxy0 + 2 * MPS) = nw;
@@ -381,22 +423,33 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
                 const float *h = ur + b * MSS + hxy1;
                 float eu, ev, ew;
                 rhs_one<CRF>(h, ur + a * MSS + hxy1, P, K, fh, eu, ev, ew);
-                o[hxy1] = h[0] + eu;
-                o[hxy1 + MPS] = h[MPS] + ev;
-                o[hxy1 + 2 * MPS] = top ? 0.f : h[2 * MPS] + ew;
+                if constexpr (WIDE) {
+                    o[hxy1] = (float)(h64[0] + (double)eu);
+                    o[hxy1 + MPS] = (float)(h64[1] + (double)ev);
+                    o[hxy1 + 2 * MPS] = top ? 0.f : (float)(h64[2] + (double)ew);
+                    eh = eu;
+                } else {
+                    o[hxy1] = h[0] + eu;
+                    o[hxy1 + MPS] = h[MPS] + ev;
+                    o[hxy1 + 2 * MPS] = top ? 0.f : h[2 * MPS] + ew;
+                }
             }
         } else if (p.whi && mq == p.nz + 1) {
             // imposeNoSlipBC on the stage-1 field: plane nz+1 from plane nz
             float *o = sr + a * MSS;
             const float *n = sr + b * MSS;
             auto image = [&](int xy) {
-                o[xy] = bcu2 - n[xy];
+                o[xy] = bcu2 - n[xy]; // exact where u_crf is zero
                 o[xy + MPS] = -n[xy + MPS];
                 o[xy + 2 * MPS] = 0.f;
             };
             image(hxy0);
             image(hxy0 + 1);
             if (hval) image(hxy1);
+            if constexpr (WIDE && CRF) { // the image in FP64
+                *reinterpret_cast<float2 *>(o + hxy0) = image32(q1[0], d1[0]);
+                if (hval) o[hxy1] = (float)((b2 - __ldg(u + sk * p.nz + swH)) - (double)eh);
+            }
         }
         // stage 2's operands from global memory, ahead of the barrier
         double2 u0 = {}, v0 = {}, w0 = {};
@@ -409,9 +462,9 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
                 qy = __ldg(reinterpret_cast<const float2 *>(q + gN));
                 qz = (kq < p.nz) ? __ldg(reinterpret_cast<const float2 *>(q + sk + gA)) : qc;
             }
-            u0 = __ldg(reinterpret_cast<const double2 *>(u + pl + gA));
-            v0 = __ldg(reinterpret_cast<const double2 *>(v + pl + gA));
-            w0 = __ldg(reinterpret_cast<const double2 *>(w + pl + gA));
+            u0 = WIDE ? e64[0] : pair64(u, pl + gA);
+            v0 = WIDE ? e64[1] : pair64(v, pl + gA);
+            w0 = WIDE ? e64[2] : pair64(w, pl + gA);
         }
         __syncthreads();
         // ring slot of plane mq, which stage 1 above has finished with
@@ -421,39 +474,58 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
             const MPlane P = m_plane(tab, kq);
             f2 du, dv, dw;
             rhs_pair2<CRF>(sr + b * MSS + hxy0, sr + a * MSS + hxy0, P, K, s2, du, dv, dw);
-            const f2 half = bc2(0.5f);
-            du = mul2(half, add2(e1[0], du));
-            dv = mul2(half, add2(e1[1], dv));
-            dw = mul2(half, add2(e1[2], dw));
-            if (pinc) {
-                du = fma2(K.ngx, sub2(pk2(qc.y, qE), qc), du);
-                dv = fma2(K.ngy, sub2(qy, qc), dv);
-                dw = fma2(bc2(P.nhw), sub2(qz, qc), dw);
-                qc = qz;
+            double2 nu, nv, nw;
+            if constexpr (WIDE) {
+                // ((q + d1) + d2 + q) / 2 - dt G p_pred
+                auto mean = [](double q, float a, float b) { return ((q + (double)a) + (double)b + q) * 0.5; };
+                nu = make_double2(mean(u0.x, e1[0].x, du.x), mean(u0.y, e1[0].y, du.y));
+                nv = make_double2(mean(v0.x, e1[1].x, dv.x), mean(v0.y, e1[1].y, dv.y));
+                nw = make_double2(mean(w0.x, e1[2].x, dw.x), mean(w0.y, e1[2].y, dw.y));
+                if (pinc) {
+                    const double gx = p.dt * p.dx_inv, gy = p.dt * p.dy_inv, gz = p.dt * __ldg(m.dzc_inv + kq);
+                    const double q0 = qc.x, q1 = qc.y;
+                    nu.x -= (q1 - q0) * gx;
+                    nu.y -= ((double)qE - q1) * gx;
+                    nv.x -= ((double)qy.x - q0) * gy;
+                    nv.y -= ((double)qy.y - q1) * gy;
+                    nw.x -= ((double)qz.x - q0) * gz;
+                    nw.y -= ((double)qz.y - q1) * gz;
+                }
+            } else {
+                const f2 half = bc2(0.5f);
+                du = mul2(half, add2(e1[0], du));
+                dv = mul2(half, add2(e1[1], dv));
+                dw = mul2(half, add2(e1[2], dw));
+                if (pinc) {
+                    du = fma2(K.ngx, sub2(pk2(qc.y, qE), qc), du);
+                    dv = fma2(K.ngy, sub2(qy, qc), dv);
+                    dw = fma2(bc2(P.nhw), sub2(qz, qc), dw);
+                }
+                nu = make_double2(u0.x + (double)du.x, u0.y + (double)du.y);
+                nv = make_double2(v0.x + (double)dv.x, v0.y + (double)dv.y);
+                nw = make_double2(w0.x + (double)dw.x, w0.y + (double)dw.y);
             }
+            if (pinc) qc = qz;
             if (inside) {
                 auto put = [&](double *f, size_t at, double x, double y) {
                     *reinterpret_cast<double2 *>(f + at + gA) = make_double2(x, y);
                 };
-                const double nu0 = u0.x + (double)du.x, nu1 = u0.y + (double)du.y;
-                const double nv0 = v0.x + (double)dv.x, nv1 = v0.y + (double)dv.y;
-                put(uo, pl, nu0, nu1);
-                put(vo, pl, nv0, nv1);
-                if (kq != p.nz || !p.whi) put(wo, pl, w0.x + (double)dw.x, w0.y + (double)dw.y);
+                put(uo, pl, nu.x, nu.y);
+                put(vo, pl, nv.x, nv.y);
+                if (kq != p.nz || !p.whi) put(wo, pl, nw.x, nw.y);
                 // imposeNoSlipBC
-                const double b2 = 2.0 * (0.0 - p.u_crf);
                 if (p.wlo && kq == 1) {
-                    put(uo, pl - sk, b2 - nu0, b2 - nu1);
-                    put(vo, pl - sk, -nv0, -nv1);
+                    put(uo, pl - sk, b2 - nu.x, b2 - nu.y);
+                    put(vo, pl - sk, -nv.x, -nv.y);
                     put(wo, pl - sk, 0.0, 0.0);
                 }
                 if (p.whi && kq == p.nz) {
-                    put(uo, pl + sk, b2 - nu0, b2 - nu1);
-                    put(vo, pl + sk, -nv0, -nv1);
+                    put(uo, pl + sk, b2 - nu.x, b2 - nu.y);
+                    put(vo, pl + sk, -nv.x, -nv.y);
                     put(wo, pl, 0.0, 0.0);
                     put(wo, pl + sk, 0.0, 0.0);
                 }
-                su += (nu0 + nu1) * pzl[kq];
+                su += (nu.x + nu.y) * pzl[kq];
             }
         } else if (kq == kbeg - 1) {
             // the bottom fluxes of stage 2's first plane: u1 plane kbeg in slot
@@ -466,7 +538,9 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
                 s2.u = u1;
                 s2.v = v1;
                 s2.w = ld2(n + 2 * MPS);
-                s2.fu = top_flux2(P, bc2(0.f), sub2(bc2(bcu2), u1), u1);
+                f2 ub = sub2(bc2(bcu2), u1);
+                if constexpr (WIDE && CRF) ub = image32(q1[0], d1[0]); // the image in FP64
+                s2.fu = top_flux2(P, bc2(0.f), ub, u1);
                 s2.fv = top_flux2(P, bc2(0.f), make_float2(-v1.x, -v1.y), v1);
                 s2.fw = w_flux2(P, bc2(0.f), ld2(n + 2 * MPS));
             } else {
@@ -475,7 +549,10 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
             if (pinc && inside) qc = __ldg(reinterpret_cast<const float2 *>(pq + gA + sk * (kbeg - 1)));
         }
 #pragma unroll
-        for (int q = 0; q < 3; q++) e1[q] = d1[q];
+        for (int q = 0; q < 3; q++) {
+            e1[q] = d1[q];
+            e64[q] = q1[q];
+        }
         __syncthreads();
     };
     const int stop = kend + 1;
@@ -487,6 +564,19 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
     }
     cp_async_wait<0>();
     mean_reduce(su, red);
+}
+
+// Grids that 32 x 16 tiles divide take the FP32 forms, the others the wide ones.
+// The line is the one that the fused step has always had: grids that do not tile
+// ran the two stage kernels, whose FP64 sums they keep.  RMS error of u, v, w after
+// the RK phase against FP64, in units of the stage kernels': 0.37, 0.91, 0.81 wide,
+// 0.58, 1.11, 0.88 with the FP32 forms (324x162x30); 324x162x150 0.223 ms
+// wide, 0.168 with the FP32 forms, 0.622 as stage kernels.
+static auto mixed_kernel(const StepParams &p)
+{
+    const bool wide = p.nx % MX != 0 || p.ny % MY != 0, crf = p.u_crf != 0.0;
+    return wide ? (crf ? k_rk_mixed<true, true> : k_rk_mixed<false, true>)
+                : (crf ? k_rk_mixed<true, false> : k_rk_mixed<false, false>);
 }
 
 static dim3 mixed_tiles(const StepParams &p) { return dim3((p.nx + MX - 1) / MX, (p.ny + MY - 1) / MY, 1); }
@@ -505,8 +595,7 @@ static size_t mixed_smem()
 
 int rk_mixed_prepare(const StepParams &p, RkLaunch *out)
 {
-    return rk_prepare(p.u_crf != 0.0 ? (const void *)k_rk_mixed<true> : (const void *)k_rk_mixed<false>, MT, mixed_smem(),
-                      mixed_tiles(p), p.nz, MX_KCHUNK, out);
+    return rk_prepare((const void *)mixed_kernel(p), MT, mixed_smem(), mixed_tiles(p), p.nz, MX_KCHUNK, out);
 }
 
 int launch_rk_mixed(const double *u, const double *v, const double *w, double *uo, double *vo, double *wo,
@@ -528,8 +617,8 @@ int launch_rk_mixed(const double *u, const double *v, const double *w, double *u
     K.ncc = both(-2.0 * p.dt * p.re_inv * (p.dx_inv * p.dx_inv + p.dy_inv * p.dy_inv));
     K.nucx = both(-0.5 * p.dt * p.u_crf * p.dx_inv);
     MeanRed r{ms.partial, ms.counter, ms.scalar, (double)p.nx, (double)p.ny, ms.vel_force};
-    PL_CUDA_TRY(launch_chained(p.u_crf != 0.0 ? k_rk_mixed<true> : k_rk_mixed<false>, l.grid, dim3(MX, MT / MX),
-                               mixed_smem(), st, u, v, w, uo, vo, wo, p, m, K, r, l.kchunk, pq, pinc));
+    PL_CUDA_TRY(launch_chained(mixed_kernel(p), l.grid, dim3(MX, MT / MX), mixed_smem(), st, u, v, w, uo, vo, wo, p, m, K,
+                               r, l.kchunk, pq, pinc));
     return 0;
 }
 
