@@ -158,7 +158,10 @@ int pl_channel_upload_compact(pl_channel *c, const double *uvw);
 int pl_channel_download_compact(pl_channel *c, double *uvw);
 /* device pointers of the current fields (for per-phase entries and tests):
  * which = 0..2 u,v,w (FP64, nx*ny*(nz+2)), 3 = p (interior), 4..6 = stage-1
- * fields u1,v1,w1 (FP64 path) or stage-1 increments (mixed path, FP32) */
+ * fields u1,v1,w1 (FP64 path) or stage-1 increments (mixed path, FP32) of the
+ * last RK phase.  Ask again after every step: u, v, w move between two sets
+ * of arrays, and 3..6 are brought up to date (on the channel's stream) by the
+ * call. */
 void *pl_channel_field(pl_channel *c, int which);
 void *pl_channel_stream(pl_channel *c);
 

@@ -453,6 +453,7 @@ int adjoint_step(pl_channel *c, const double *xu, const double *xv, const double
     double *cu = W.y1, *cv = W.y1 + nf, *cw = W.y1 + 2 * nf;
     // stage-1 state y1 = RK1(x) (with its wall fill) into u1, v1, w1
     if (launch_rk1_fp64(xu, xv, xw, c->u1, c->v1, c->w1, p, c->m, st)) return -1;
+    c->stage1_stale = false;
     // forceVel^T, W^-1
     const int fx = c->cfg.is_forced[0];
     if (fx && level_sums(0, au, av, aw, c, W.part, 1.0, 0, W.scal)) return -1;

@@ -518,8 +518,23 @@ const double *pl::channel_p64(pl_channel *c)
 // correction uses the FP32 increment alone.
 static int mixed_incremental(const pl_channel *c) { return (c->incremental && c->nsolve >= 2) ? 1 : 0; }
 
+// The fused RK kernel keeps the stage-1 field on chip: what readers and a lone
+// second stage see of it is formed from that phase's input when they ask.
+static int stage1_refresh(pl_channel *c)
+{
+    if (!c->stage1_stale) return 0;
+    StepParams p = c->sp;
+    std::memcpy(p.fb, c->stage1_fb, sizeof(p.fb));
+    if (is_mixed(c) ? launch_rk1_mixed(c->ub, c->vb, c->wb, c->d1u, c->d1v, c->d1w, p, c->m, c->stream)
+                    : launch_rk1_fp64(c->ub, c->vb, c->wb, c->u1, c->v1, c->w1, p, c->m, c->stream))
+        return -1;
+    c->stage1_stale = false;
+    return 0;
+}
+
 extern "C" int pl_phase_rk1(pl_channel *c)
 {
+    c->stage1_stale = false;
     int rc = is_mixed(c) ? launch_rk1_mixed(c->u, c->v, c->w, c->d1u, c->d1v, c->d1w, c->sp, c->m, c->stream)
                          : launch_rk1_fp64(c->u, c->v, c->w, c->u1, c->v1, c->w1, c->sp, c->m, c->stream);
     channel_mark(c, "rk1");
@@ -528,6 +543,7 @@ extern "C" int pl_phase_rk1(pl_channel *c)
 
 extern "C" int pl_phase_rk2(pl_channel *c)
 {
+    if (stage1_refresh(c)) return -1;
     int rc;
     if (is_mixed(c)) {
         rc = launch_rk2_mixed(c->u, c->v, c->w, c->d1u, c->d1v, c->d1w, c->ub, c->vb, c->wb, c->sp, c->m, c->ms,
@@ -631,6 +647,8 @@ extern "C" int pl_phase_rk(pl_channel *c)
     std::swap(c->u, c->ub);
     std::swap(c->v, c->vb);
     std::swap(c->w, c->wb);
+    c->stage1_stale = c->u1 != nullptr || c->d1u != nullptr; // a slab has none
+    std::memcpy(c->stage1_fb, c->sp.fb, sizeof(c->stage1_fb));
     channel_mark(c, "rk_fused");
     return rc;
 }
@@ -762,6 +780,10 @@ extern "C" int pl_channel_get_field(pl_channel *c, int which, double *host)
         set_error("pl_channel_get_field: which must be 0..6");
         return -1;
     }
+    if (which >= 4) {
+        if (stage1_refresh(c)) return -1;
+        PL_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    }
     std::vector<double> tmp(c->nf);
     if (which == 3) {
         channel_p64(c);
@@ -827,6 +849,7 @@ extern "C" int pl_channel_download_compact(pl_channel *c, double *uvw)
 
 extern "C" void *pl_channel_field(pl_channel *c, int which)
 {
+    if (which >= 4 && which <= 6 && stage1_refresh(c)) return nullptr;
     switch (which) {
     case 0: return c->u;
     case 1: return c->v;

@@ -26,7 +26,7 @@ struct pl_channel {
     pl::MeshDev m{};
     // FP64 path: u,v,w = ua,va,wa; stage-1 fields u1,v1,w1; p
     // mixed path: u,v,w ping-pong between (ua,va,wa) and (ub,vb,wb); stage-1
-    // increments d1u,d1v,d1w (FP32, the per-phase entries only); p32 = p_n
+    // increments d1u,d1v,d1w (FP32; the per-phase entries, and on demand); p32 = p_n
     // (FP32, updated in place by the solve); the pressure prediction for the
     // next projection in pm32, written into pb32 by the solve and swapped;
     // the PPE works in place on r32 (FP32); p (FP64) is p32 widened on demand
@@ -37,6 +37,10 @@ struct pl_channel {
     double *ub = nullptr, *vb = nullptr, *wb = nullptr;
     float *p32 = nullptr, *pm32 = nullptr, *pb32 = nullptr;
     bool p_stale = false; // mixed: p lags p32
+    // the stage-1 fields lag the last RK phase, whose input is in ub, vb, wb and
+    // whose body force was stage1_fb (stage1_refresh)
+    bool stage1_stale = false;
+    double stage1_fb[3] = {0.0, 0.0, 0.0};
     float *d1u = nullptr, *d1v = nullptr, *d1w = nullptr, *r32 = nullptr;
     double *plane_part = nullptr, *mode0 = nullptr;
     int incremental = 1;   // mixed path: solve for a pressure increment (Thomas)

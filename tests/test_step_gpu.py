@@ -256,3 +256,48 @@ def test_step_matches_phases(gpu, precision, nx, ny, nz):
         assert max(errs) < 1e-11
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny,nz", [(24, 18, 12), (32, 16, 8)])
+def test_stage_one_fields_after_a_step(gpu, precision, nx, ny, nz):
+    """Fields 4..6 after pl_channel_step are the stage-1 fields (mixed: increments) of its last
+    RK phase, those of pl_phase_rk1 from the same state bit for bit, although the step's kernel
+    keeps them on chip; a body force that is set later does not enter them."""
+    import torch
+    plb = gpu
+    cfg = plb.ChannelConfig(nx=nx, ny=ny, nz=nz, stretch_ratio=1.5, re_tau=180.0, dt=1e-3,
+                            precision=plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED)
+
+    class View:
+        def __init__(self, ptr):
+            self.__cuda_array_interface__ = {"data": (ptr, False), "shape": (nz + 2, ny, nx), "version": 2,
+                                             "typestr": "<f8" if precision == "fp64" else "<f4"}
+
+    def stage_one(ch):
+        out = []
+        for which in (4, 5, 6):
+            ptr = ch.field_ptr(which)
+            ch.synchronize()
+            out.append(torch.as_tensor(View(ptr), device="cuda").cpu().numpy())
+        return out
+
+    a, b = plb.Channel(cfg), plb.Channel(cfg)
+    for ch in (a, b):
+        ch.init_flow(3, 0.1)
+        if precision == "fp64":
+            ch.set_body_force((0.2, 0.0, 0.1))
+        ch.step(2)
+    a.step(1)
+    if precision == "fp64":
+        a.set_body_force((0.0, 0.5, 0.0))
+    b.phase("rk1")
+    want = stage_one(b)
+    assert want[0].any()
+    for x, y in zip(stage_one(a), want):
+        assert np.array_equal(x, y)
+    if precision == "fp64":
+        for which in (4, 5, 6):
+            assert np.array_equal(a.get_field(which), b.get_field(which))
+    a.close()
+    b.close()
