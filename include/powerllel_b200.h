@@ -210,7 +210,8 @@ int pl_adjoint_ke_gradient(pl_channel *c, int nsteps, int every, double *ke, dou
 /* ======================================================================
  * 6. Statistics and monitors (src/mod_statistics.f90, src/mod_monitor.f90),
  *    computed on the device; the reference writes them to text and HDF5
- *    files, here the caller receives the values.
+ *    files, here the caller receives the values.  Between steps, several
+ *    threads may read one channel's monitors, kinetic energy and diagnostics.
  * ====================================================================== */
 /* bits of `which`, in the order of stat_which_var: */
 #define PL_STAT_U (1u << 0)

@@ -499,6 +499,7 @@ extern "C" int pl_channel_set_body_force(pl_channel *c, const double f[3])
 
 extern "C" int pl_channel_kinetic_energy(pl_channel *c, double *ke)
 {
+    std::lock_guard<std::mutex> lk(c->mon_mu);
     double *out = c->d_mon;
     int rc = level_sums(1, c->u, c->v, c->w, c, c->d_mon + MON_OUT, 1.0, 0, out);
     double h[3] = {0, 0, 0};

@@ -713,6 +713,7 @@ extern "C" int pl_channel_synchronize(pl_channel *c)
 
 extern "C" int pl_channel_diagnostics(pl_channel *c, pl_diag *out)
 {
+    std::lock_guard<std::mutex> lk(c->mon_mu);
     int *d_loc = reinterpret_cast<int *>(c->d_diag + 4);
     if (launch_diagnostics_fp64(c->u, c->v, c->w, c->sp, c->m, c->d_diag, d_loc, c->d_dpart, c->d_dipart, c->max_blocks,
                                 c->stream))

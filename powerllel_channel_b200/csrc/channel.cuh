@@ -2,6 +2,7 @@
 // entry points, shared by the step (channel.cu) and its adjoint (adjoint.cu).
 #pragma once
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -50,7 +51,10 @@ struct pl_channel {
     pl::MeanState ms;
     pl::RkLaunch rk;
     double *d_diag = nullptr; // [0..3] values, [4..] the locations (int)
-    // the monitors' and the kinetic energy's scratch: results, then partial sums
+    // the monitors' and the kinetic energy's scratch: results, then partial sums;
+    // held by mon_mu from the launch to the copy of the result, so that threads
+    // reading one channel do not overwrite each other's
+    std::mutex mon_mu;
     double *d_mon = nullptr;
     unsigned int *d_mon_count = nullptr; // zero between launches
     void *adj = nullptr;                 // the adjoint's fields and checkpoints (adjoint.cu), once used

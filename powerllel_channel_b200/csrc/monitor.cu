@@ -252,6 +252,7 @@ extern "C" int pl_monitor_skin_friction(pl_channel *c, int wall, double *u_tau, 
     // calcAndWriteSkf (:264-296): tau_w = mean of re_inv (u(k_wall) + u_crf) / dz,
     // dz = dzf(k_wall)/2, k_wall = 1 or nz
     const int kw = wall == 0 ? 1 : c->nz;
+    std::lock_guard<std::mutex> lk(c->mon_mu);
     double sum = 0.0;
     k_planes_sum<<<dim3(64, 1), 256, 0, c->stream>>>(c->u, kw, nullptr, c->sp, c->d_mon + MON_OUT, c->d_mon_count,
                                                      c->d_mon);
@@ -271,6 +272,7 @@ extern "C" int pl_monitor_skin_friction(pl_channel *c, int wall, double *u_tau, 
 extern "C" int pl_monitor_forcing(pl_channel *c, double vel_mean[3])
 {
     // calcAndWriteForcing (:298-318): Mean_h of the forced components, u_crf added to u
+    std::lock_guard<std::mutex> lk(c->mon_mu);
     const double *f[3] = {c->u, c->v, c->w};
     for (int d = 0; d < 3; d++) {
         vel_mean[d] = 0.0;
@@ -297,6 +299,7 @@ extern "C" int pl_monitor_probe(pl_channel *c, int i, int j, int k, double out[4
     }
     const size_t sk = (size_t)c->nx * c->ny;
     const size_t g = (size_t)(i - 1) + (size_t)c->nx * (j - 1) + sk * k;
+    std::lock_guard<std::mutex> lk(c->mon_mu);
     k_probe<<<1, 1, 0, c->stream>>>(c->u, c->v, c->w, state_p(c), g, g - sk, c->d_mon);
     PL_CHECK_LAUNCH();
     PL_CUDA_TRY(cudaMemcpyAsync(out, c->d_mon, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

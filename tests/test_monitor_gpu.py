@@ -78,3 +78,20 @@ def test_monitors_match_numpy(gpu):
     with pytest.raises(plb.PowerLLELError):
         ch.probe(0, 1, 1)
     ch.close()
+
+
+def test_monitors_read_by_two_threads(gpu):
+    """Threads that read the monitors of one channel get their own results."""
+    from concurrent.futures import ThreadPoolExecutor
+    plb = gpu
+    ch = plb.Channel(plb.ChannelConfig(nx=64, ny=48, nz=32, stretch_ratio=1.5, re_tau=180.0))
+    ch.init_flow(5, 0.1)
+    ch.step(2)
+    reads = [lambda: ch.skin_friction(0), lambda: ch.skin_friction(1), lambda: ch.forcing_means()[0], ch.kinetic_energy,
+             lambda: tuple(ch.probe(7, 11, 13)), lambda: tuple(ch.probe(9, 3, 20))]
+    want = [r() for r in reads]
+    assert len(set(map(str, want))) == len(want)
+    with ThreadPoolExecutor(len(reads)) as pool:
+        wrong = list(pool.map(lambda q: sum(reads[q]() != want[q] for _ in range(300)), range(len(reads))))
+    assert wrong == [0] * len(reads)
+    ch.close()
