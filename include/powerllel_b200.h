@@ -201,10 +201,15 @@ int pl_channel_kinetic_energy(pl_channel *c, double *ke);
  * wall planes and w's level nz zero) and dJ/df to grad_f (host).  The
  * gradient is with respect to the degrees of freedom: u, v on levels 1..nz,
  * w on levels 1..nz-1.  On return u, v, w hold x0 again; p and the stage-1
- * fields are overwritten.  Device memory: (ceil(nsteps/every) + every + 9)
- * fields, kept with the channel until it is destroyed.  Errors: mixed precision, PDD (trid_parts > 1), nsteps < 0, every < 1. */
+ * fields are overwritten.  Device memory: 3 (max(1, ceil(nsteps/every)) +
+ * min(every, max(1, nsteps))) + 9 fields, in one allocation.  It stays with the
+ * channel for the next call where all channels of the process then keep at
+ * most 1/32 of the device's memory so, and is freed on return otherwise.
+ * Errors: mixed precision, PDD (trid_parts > 1), nsteps < 0, every < 1. */
 int pl_adjoint_ke_gradient(pl_channel *c, int nsteps, int every, double *ke, double *d_gu, double *d_gv,
                            double *d_gw, double grad_f[3]);
+/* frees the device memory that the gradient keeps with the channel */
+int pl_adjoint_release(pl_channel *c);
 
 
 /* ======================================================================

@@ -102,6 +102,7 @@ def lib():
     L.pl_channel_set_body_force.argtypes = [C.c_void_p, _dp]
     L.pl_channel_kinetic_energy.argtypes = [C.c_void_p, _dp]
     L.pl_adjoint_ke_gradient.argtypes = [C.c_void_p, C.c_int, C.c_int, _dp, C.c_void_p, C.c_void_p, C.c_void_p, _dp]
+    L.pl_adjoint_release.argtypes = [C.c_void_p]
     L.pl_stat_enable.argtypes = [C.c_void_p, C.c_uint, C.c_int, C.c_int]
     L.pl_stat_init.argtypes = [C.c_void_p]
     L.pl_stat_sample.argtypes = [C.c_void_p, C.c_int]
@@ -347,6 +348,10 @@ class Channel:
         _check(lib().pl_adjoint_ke_gradient(self._h, int(nsteps), int(every), _ptr(ke), C.c_void_p(g[0]),
                                             C.c_void_p(g[1]), C.c_void_p(g[2]), _ptr(gf)), "pl_adjoint_ke_gradient")
         return float(ke[0]), gf
+
+    def adjoint_release(self) -> None:
+        """Free the device memory that adjoint_ke_gradient keeps with the channel."""
+        _check(lib().pl_adjoint_release(self._h), "pl_adjoint_release")
 
     # statistics (mod_statistics.f90) -------------------------------------
     STAT_NAMES = ("u", "v", "w", "u2", "v2", "w2", "uv", "uw", "vw", "p", "p2")

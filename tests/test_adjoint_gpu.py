@@ -190,3 +190,37 @@ def test_adjoint_rejects_mixed_and_pdd(gpu):
     with pytest.raises(plb.PowerLLELError, match="Thomas"):
         ch.adjoint_ke_gradient(2, 1, g.data_ptr(), g.data_ptr(), g.data_ptr())
     ch.close()
+
+
+def test_adjoint_keeps_a_bounded_workspace(gpu):
+    """What a call leaves allocated is at most 1/32 of the device's memory, whatever it used (here
+    130 fields of 51 MB), is not more after calls of opposite shapes than the larger one needs, and
+    pl_adjoint_release gives it back; the results do not depend on what was kept."""
+    plb = gpu
+    nx, ny, nz = 256, 192, 128
+    _, ch = _mesh_and_channel(plb, nx, ny, nz, 1.8, 1000.0, 1e-4, 7, 0.05)
+    g = [torch.zeros((nz + 2, ny, nx), dtype=torch.float64, device="cuda") for _ in range(3)]
+    field = 8 * nx * ny * (nz + 2)
+
+    def call(nsteps, every):
+        J, gf = ch.adjoint_ke_gradient(nsteps, every, *(t.data_ptr() for t in g))
+        torch.cuda.synchronize()
+        return J, gf.copy(), [t.cpu() for t in g]
+
+    def same(a, b):
+        return a[0] == b[0] and np.array_equal(a[1], b[1]) and all(torch.equal(x, y) for x, y in zip(a[2], b[2]))
+
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    slack = 64 << 20  # what the driver rounds and loads
+    one = call(8, 1)     # 8 checkpoints, 1 state: 36 fields with the nine
+    other = call(8, 8)   # 1 checkpoint, 8 states
+    assert free - torch.cuda.mem_get_info()[0] <= 36 * field + slack
+    assert same(call(8, 1), one) and same(call(8, 8), other)
+    call(40, 1)          # 41 states
+    assert free - torch.cuda.mem_get_info()[0] <= total // 32 + slack
+    assert same(call(8, 1), one)
+    ch.adjoint_release()
+    assert free - torch.cuda.mem_get_info()[0] <= slack
+    assert same(call(8, 8), other)
+    ch.close()
