@@ -50,7 +50,7 @@ def _relmax(a, b):
     return float(np.abs(a - b).max() / np.abs(b).max())
 
 
-@pytest.mark.parametrize("grid", [(32, 24, 16), (24, 18, 12)])  # fused RK kernel / separate RK1, RK2 kernels
+@pytest.mark.parametrize("grid", [(32, 24, 16), (24, 18, 12)])  # whole tiles / tiles past the domain
 def test_body_force_step_matches_reference(gpu, grid):
     plb = gpu
     nx, ny, nz = grid
@@ -223,4 +223,30 @@ def test_adjoint_keeps_a_bounded_workspace(gpu):
     ch.adjoint_release()
     assert free - torch.cuda.mem_get_info()[0] <= slack
     assert same(call(8, 8), other)
+    ch.close()
+
+
+@pytest.mark.parametrize("u_crf", [0.0, 0.3])
+@pytest.mark.parametrize("nx,ny,nz,nsteps,every", [(24, 18, 12, 4, 2), (54, 36, 10, 3, 3), (6, 4, 2, 4, 1), (96, 12, 66, 2, 1)])
+def test_adjoint_on_ragged_grids_matches_autograd_reference(gpu, nx, ny, nz, nsteps, every, u_crf):
+    """The transposed stencil where its 32 x 8 tiles reach past the domain, are wider than it, and
+    wrap; with and without the moving frame's terms; chunks of two planes and of the whole column."""
+    plb = gpu
+    ch = plb.Channel(plb.ChannelConfig(nx=nx, ny=ny, nz=nz, stretch_ratio=1.8, re=200.0, dt=1e-3, u_crf=u_crf))
+    ch.init_flow(5, 0.3)
+    m = A.Mesh(nx, ny, nz, stretch=1.8, re=200.0, dt=1e-3, u_crf=u_crf)
+    f = np.array([0.3, 0.1, -0.2])
+    ch.set_body_force(f)
+    x0 = _download(ch)
+    g = [torch.zeros((nz + 2, ny, nx), dtype=torch.float64, device="cuda") for _ in range(3)]
+    J, gf = ch.adjoint_ke_gradient(nsteps, every, *(t.data_ptr() for t in g))
+    torch.cuda.synchronize()
+    K = slice(1, nz + 1)
+    Jr, gu, gv, gw, gfr = A.gradient(m, x0[0][K], x0[1][K], x0[2][K], f, nsteps)
+    got = [t.cpu().numpy() for t in g]
+    errs = [_relmax(got[c][K], r) for c, r in enumerate((gu, gv, gw))]
+    print(f"{nx}x{ny}x{nz} u_crf {u_crf}: J rel {abs(J - Jr) / abs(Jr):.2e} grad rel max {errs}", gf, gfr)
+    assert abs(J - Jr) <= 1e-12 * abs(Jr)
+    assert max(errs) < 1e-9
+    assert np.abs(gf - gfr).max() <= 1e-9 * np.abs(gfr).max()
     ch.close()

@@ -108,3 +108,44 @@ def test_step_matches_phases(gpu, precision, nx, ny, nz):
             assert np.abs(x - y).max() < 1e-11 * np.abs(y).max()
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("nz", [1016, 1022, 1024, 1026, 1032])
+def test_solve_by_tall_column(gpu, oracle_mod, nz, precision, tol):
+    """Around the 1,024 rows up to which the sweep uses tensor memory: above them its values are
+    swept through device memory alone."""
+    plb, O = gpu, oracle_mod
+    g, r, ref = rhs_and_reference(O, 16, 18, nz)
+    got = solve(plb, g, r, plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED)
+    assert np.abs(got - ref).max() < tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("nx,ny,nz,nparts,precision", [
+    (512, 384, 192, 8, "mixed"),                                 # batches of 8 rows, one column a thread
+    (192, 162, 576, 4, "fp64"), (288, 216, 576, 4, "mixed"),     # 16 rows, one column: 144 rows a partition
+    (512, 384, 96, 3, "fp64"), (512, 384, 192, 4, "mixed")])     # 16 rows, two columns
+def test_pdd_variants_on_arrays_larger_than_l2(gpu, oracle_mod, nx, ny, nz, nparts, precision):
+    """143 to 151 MB: the variants of the partition sweep that request the next batch of rows into L2."""
+    plb, O = gpu, oracle_mod
+    g, r, ref = rhs_and_reference(O, nx, ny, nz, nparts)
+    got = solve(plb, g, r, plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED, nparts)
+    assert np.abs(got - ref).max() < (1e-12 if precision == "fp64" else 1e-5) * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("nparts", [0, 3])
+@pytest.mark.parametrize("n", LENGTHS)
+def test_host_solve_by_line_length(gpu, oracle_mod, n, nparts):
+    """init/execute/free_poisson_solver: the strided x transforms of every length on the ghosted
+    host array, whose ghosts stay untouched.  The FP64 bar."""
+    plb, O = gpu, oracle_mod
+    ny, nz = LENGTHS[(LENGTHS.index(n) + 1) % 6], 12
+    g, r, ref = rhs_and_reference(O, n, ny, nz, nparts)
+    var = np.full((nz + 2, ny + 2, n + 2), 7.25)
+    var[1:-1, 1:-1, 1:-1] = r
+    with plb.PoissonSolver(n, ny, nz, g.g.dx, g.g.dy, g.dzf_global, nparts=nparts) as s:
+        s.execute(var)
+    got = var[1:-1, 1:-1, 1:-1].copy()
+    var[1:-1, 1:-1, 1:-1] = 7.25
+    assert np.all(var == 7.25)
+    assert np.abs((got - got.mean()) - ref).max() < 1e-12 * np.abs(ref).max()

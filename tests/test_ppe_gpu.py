@@ -91,11 +91,12 @@ def test_device_ppe_vs_golden(gpu, path):
     assert torch.equal(x, y)
 
 
-# Thomas keeps its swept values in tensor memory for nz % 8 == 0: all of them
-# for nz <= 256 (768x32x256: two rounds of columns per CTA; 16x8x8: one 8-row
-# group, exactly one CTA of 128 columns; 8x6x16: one CTA with 80 idle
-# threads), 256 of them for taller columns with the rest in HBM (32x24x264,
-# 32x24x512); in HBM alone for other nz.  PDD: each partition in tensor
+# Thomas keeps its swept values in tensor memory: all of them for nz <= 256
+# (768x32x256: two rounds of columns per CTA; 16x8x8: one 8-row group, exactly
+# one CTA of 128 columns; 8x6x16: one CTA with 80 idle threads; 64x48x30: a
+# last group of 6 rows), 256 of them for taller columns with the rest in HBM
+# (32x24x264, 32x24x512), in HBM alone from 1,026 rows on
+# (test_line_lengths_gpu).  PDD: each partition in tensor
 # memory for up to 8 partitions of multiples of 8 rows (256x192x32/4,
 # 64x48x32/2), one thread per (column, partition) with the swept values in
 # HBM otherwise up to 32 partitions (64x48x40/8, 96x72x30/4, 32x24x96/12,
