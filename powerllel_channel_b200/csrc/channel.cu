@@ -371,8 +371,7 @@ static int channel_create(pl_channel **out, const pl_channel_config *cfg, int zr
         return true;
     };
     if (zn > 1 && (c->nx % 32 != 0 || c->ny % (mixed ? 16 : 8) != 0)) {
-        set_error("pl_channel_create_slab: the slab step needs the fused RK kernel: nx % 32 == 0 and ny % 8 == 0 "
-                  "(FP64) or ny % 16 == 0 (mixed)");
+        set_error("pl_channel_create_slab: z slabs take nx % 32 == 0 and ny % 8 == 0 (FP64) or ny % 16 == 0 (mixed)");
         return fail();
     }
     // velocity-like fields with hx halo planes beyond each wall plane

@@ -84,3 +84,19 @@ def test_slabs_match_one_gpu_pdd(gpu, precision, nx, ny, nz, G):
         assert max(l2) <= 1e-5
     for s in slabs:
         s.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz,G", [(64, 24, 32, 2), (32, 8, 24, 3)])
+def test_slabs_with_half_a_tile_in_y_match_one_gpu_pdd(gpu, nx, ny, nz, G):
+    """FP64 slabs take ny % 8 == 0: the RK kernel's last tile row reaches past the domain."""
+    test_slabs_match_one_gpu_pdd(gpu, "fp64", nx, ny, nz, G)
+
+
+@pytest.mark.parametrize("precision,nx,ny", [("fp64", 48, 16), ("fp64", 32, 36), ("mixed", 32, 24)])
+def test_slab_grid_limits(gpu, precision, nx, ny):
+    plb = gpu
+    from powerllel_channel_b200 import slab as S
+    cfg = plb.ChannelConfig(nx=nx, ny=ny, nz=16, trid_parts=2,
+                            precision=plb.PL_FP64 if precision == "fp64" else plb.PL_MIXED)
+    with pytest.raises(plb.PowerLLELError, match="z slabs take nx % 32 == 0"):
+        S.Slab(cfg, 0, 2)
