@@ -1109,7 +1109,6 @@ __global__ void __launch_bounds__(1024) k_pdd_par(const T *xin, double *xs, T *x
 // last local values meet in shared memory for the interface systems.  The
 // values are k_pdd's, expression for expression.
 constexpr int PTM_G = 8;
-constexpr size_t L2_BYTES = (size_t)126 << 20;
 
 __host__ __device__ constexpr int pdd_tm_static_smem(int nc) { return nc * 2 * 8 * 32 * 8 + 16; }
 
@@ -1568,6 +1567,10 @@ int ppe_create(Ppe *s, int nx, int ny, int nz, double dx, double dy, const doubl
         PL_CUDA_TRY(cudaMalloc(&s->d_scratch, sizeof(double) * s->scratch_elems));
     }
     if (prec == PREC_FP64 ? prepare_ct<double>(s) : prepare_ct<float>(s)) return -1;
+    int dev = 0, l2 = 0;
+    PL_CUDA_TRY(cudaGetDevice(&dev));
+    PL_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+    s->l2_bytes = (size_t)l2;
     // kernels with > 48 KB of dynamic shared memory
     PL_CUDA_TRY(cudaFuncSetAttribute(k_yfft<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     PL_CUDA_TRY(cudaFuncSetAttribute(k_yfft<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -1843,9 +1846,9 @@ template <typename T> static int launch_trid(Ppe *s, T *x, cudaStream_t st, cons
             // (one column against two per thread, us, mixed: 256x192x128 P 4
             // 38.8, 30.9; 512x384x256 P 8 390, 267, P 4 326, 255; 64x64x64 P 4
             // 9.9, 10.4 on 66 CTAs; 256x192x256 P 8 75.6, 79.4).
-            const bool pf = sizeof(T) * (size_t)ncol * s->nz > L2_BYTES;
+            const bool pf = sizeof(T) * (size_t)ncol * s->nz > s->l2_bytes;
             const int pairs = s->nx * (s->ny / 2 + 1);
-            const int nc = groups2 && 2 * cells <= 512 && pairs >= 32 * 148 &&
+            const int nc = groups2 && 2 * cells <= 512 && pairs >= 32 * sm_count() &&
                                    (pf || s->nparts <= 4 || 2 * cells > 256) ? 2 : 1;
             while (tcols < (uint32_t)(nc * cells)) tcols *= 2;
             const int per_sm = std::max(1, std::min(512 / (int)tcols, 2048 / (32 * s->nparts)));

@@ -65,6 +65,7 @@ struct Ppe {
     // kernels, found once): x forward, inverse, inverse with the pressure
     // update, calcRHS + forward; y forward, inverse
     int grid_x[4] = {0, 0, 0, 0}, grid_y[2] = {0, 0};
+    size_t l2_bytes = 0; // of the plan's device
 
     // optional per-launch marker (profiling): called after every kernel launch
     void (*mark)(void *ctx, const char *name) = nullptr;
