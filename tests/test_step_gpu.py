@@ -301,3 +301,15 @@ def test_stage_one_fields_after_a_step(gpu, precision, nx, ny, nz):
             assert np.array_equal(a.get_field(which), b.get_field(which))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz,nparts", [(64, 64, 64, 0), (512, 384, 16, 0), (64, 48, 32, 4)])
+def test_bench_counts_the_launches_of_a_step(gpu, nx, ny, nz, nparts):
+    """bench.py's launches per step are the launch slots of pl_channel_profile."""
+    import bench
+    plb = gpu
+    for prec, name in ((plb.PL_FP64, "fp64"), (plb.PL_MIXED, "mixed")):
+        ch = plb.Channel(plb.ChannelConfig(nx=nx, ny=ny, nz=nz, trid_parts=nparts, precision=prec))
+        ch.init_flow(3, 0.1)
+        assert len(ch.profile(2)) == bench.LAUNCHES[name]
+        ch.close()
