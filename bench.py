@@ -94,7 +94,9 @@ def peaks():
 
 def traffic_from_profiles(kernel):
     """dram read+write bytes per launch of `kernel` from the committed ncu
-    summary (profiles/dram_traffic_512x384x256.txt), else None."""
+    summary (profiles/dram_traffic_512x384x256.txt) at that grid, else None."""
+    if (NX, NY, NZ) != (512, 384, 256):
+        return None
     p = os.path.join(ROOT, "profiles", "dram_traffic_512x384x256.txt")
     if not os.path.exists(p):
         return None

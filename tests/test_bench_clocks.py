@@ -54,3 +54,12 @@ def test_clock_sampler_reason_names():
     import bench
     assert bench.ClockSampler.REASON_BITS == {"sw_power_cap": 0x4, "hw_slowdown": 0x8,
                                               "sw_thermal_slowdown": 0x20, "hw_thermal_slowdown": 0x40}
+
+
+def test_measured_traffic_belongs_to_its_grid(monkeypatch):
+    """roofline.traffic is the committed DRAM measurement of the 512x384x256 kernels: no number at
+    another grid."""
+    import bench
+    assert bench.traffic_from_profiles("rk_fused") > 2.6e9
+    monkeypatch.setattr(bench, "NZ", 128)
+    assert bench.traffic_from_profiles("rk_fused") is None
