@@ -490,6 +490,7 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
                     nv.y -= ((double)qy.y - q1) * gy;
                     nw.x -= ((double)qz.x - q0) * gz;
                     nw.y -= ((double)qz.y - q1) * gz;
+                    qc = qz;
                 }
             } else {
                 const f2 half = bc2(0.5f);
@@ -500,13 +501,15 @@ __global__ void __launch_bounds__(MT, 2) k_rk_mixed(const double *__restrict__ u
                     du = fma2(K.ngx, sub2(pk2(qc.y, qE), qc), du);
                     dv = fma2(K.ngy, sub2(qy, qc), dv);
                     dw = fma2(bc2(P.nhw), sub2(qz, qc), dw);
+                    qc = qz;
                 }
-                nu = make_double2(u0.x + (double)du.x, u0.y + (double)du.y);
-                nv = make_double2(v0.x + (double)dv.x, v0.y + (double)dv.y);
-                nw = make_double2(w0.x + (double)dw.x, w0.y + (double)dw.y);
             }
-            if (pinc) qc = qz;
             if (inside) {
+                if constexpr (!WIDE) {
+                    nu = make_double2(u0.x + (double)du.x, u0.y + (double)du.y);
+                    nv = make_double2(v0.x + (double)dv.x, v0.y + (double)dv.y);
+                    nw = make_double2(w0.x + (double)dw.x, w0.y + (double)dw.y);
+                }
                 auto put = [&](double *f, size_t at, double x, double y) {
                     *reinterpret_cast<double2 *>(f + at + gA) = make_double2(x, y);
                 };
