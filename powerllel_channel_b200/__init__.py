@@ -406,6 +406,9 @@ class Channel:
         return out
 
     def field_ptr(self, which: int) -> int:
+        """Device address of a field (numbered as for get_field; mixed 4..6 are
+        FP32 increments).  Ask again after every step: u, v, w move between two
+        sets of arrays, and 3..6 are brought up to date by the call."""
         return lib().pl_channel_field(self._h, which)
 
     def profile(self, nsteps: int = 3) -> list:

@@ -61,7 +61,8 @@ dim3 adj_grid(const StepParams &p) { return dim3((p.nx + 63) / 64, (p.ny + 3) / 
 // as do the values above, the next plane's centre values: 30 shared loads a
 // point.  A kernel of a point per thread, reading its 47 operands from L1 and
 // L2, took 280 us at 256x192x128; this one takes 149, and 186 with the second
-// operand e (4.1 and 3.9 TB/s at 96 and 120 B/point).
+// operand e (3.0 and 3.2 TB/s at 72 and 96 B/point: six fields read and three
+// written, and e).
 constexpr int AX = 32, AY = 8, AW = AX + 4, AH = AY + 4, APS = AW * AH, AT = AX * AY, ASS = 6 * APS;
 
 __global__ void __launch_bounds__(AT, 2) k_adj_rk(const double *__restrict__ u, const double *__restrict__ v,

@@ -103,7 +103,8 @@ __device__ __forceinline__ void pressure_update_staged(const PressureUpdate &pu,
 // Short lines take more columns, so that a stage has work for the 256 threads.
 // Long lines take whole 64-byte row segments at one CTA per SM rather than
 // parts of them at two: FP32 at 1024x768x512, ny = 768, 4 -> 8 columns 1.015
-// -> 0.868 ms forward, 1.026 -> 0.892 ms inverse.
+// -> 0.868 ms forward, 1.026 -> 0.892 ms inverse.  FP64 lines of 432 to 512
+// take two columns, 32-byte segments; no wider choice was measured there.
 template <typename V, int N, bool FWD> __host__ __device__ constexpr int pf_y_cols()
 {
     constexpr bool fp32 = sizeof(V) == 8;

@@ -212,7 +212,7 @@ def test_adjoint_keeps_a_bounded_workspace(gpu):
 
     torch.cuda.synchronize()
     free, total = torch.cuda.mem_get_info()
-    slack = 64 << 20  # what the driver rounds and loads
+    slack = 64 << 20  # what the CUDA driver rounds up and loads
     one = call(8, 1)     # 8 checkpoints, 1 state: 36 fields with the nine
     other = call(8, 8)   # 1 checkpoint, 8 states
     assert free - torch.cuda.mem_get_info()[0] <= 36 * field + slack
